@@ -161,10 +161,10 @@ class SparseMM(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             w_csr = ctx.w_csr if ctx.w_csr is not None else _csr_weights_cached(layout, w_canon)
             gx = torch.empty_like(x)
-            gT = torch.empty(max(1, B * layout.n_out), device=g.device, dtype=torch.float32)
-            L.check(L.lib().bt_spmv_grad_input_t(B, n_in, layout.n_out, layout.csr_ptr.data_ptr(),
-                                                 layout.csr_dst.data_ptr(), w_csr.data_ptr(), g.data_ptr(),
-                                                 gx.data_ptr(), gT.data_ptr(), s), "bt_spmv_grad_input_t")
+            gT = torch.empty(max(1, (B + 3) // 4 * 4 * layout.n_out), device=g.device, dtype=torch.float32)
+            L.check(L.lib().bt_spmv_grad_input_pad(B, n_in, layout.n_out, layout.csr_ptr.data_ptr(),
+                                                   layout.csr_dst.data_ptr(), w_csr.data_ptr(), g.data_ptr(),
+                                                   gx.data_ptr(), gT.data_ptr(), s), "bt_spmv_grad_input_pad")
         if ctx.needs_input_grad[1] and layout.nnz == 0:
             gw = torch.zeros(0, device=g.device, dtype=torch.float32)
         elif ctx.needs_input_grad[1]:

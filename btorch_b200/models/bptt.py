@@ -14,7 +14,7 @@ hand-written backward kernels:
                       I_t = psc_{t-1} + P_t                  (rnn.py:524)
                       z_t, v_t, gk_t = neuron(I_t, v_{t-1}, gk_{t-1})
                       psc_t = psc_{t-1} + coef*((-psc_{t-1})/tau) + W z_t
-    backward, step t: dz_t  = gZ_t + W^T dpsc_t               (bt_spmv_grad_input_t)
+    backward, step t: dz_t  = gZ_t + W^T dpsc_t               (bt_spmv_grad_input_pad)
                       dI_t, dv_{t-1}, dgk_{t-1} = neuron'(dz_t, dv_t, dgk_t)
                       dpsc_{t-1} = dpsc_t + coef*((-dpsc_t)/tau) + dI_t   (bt_psc_step)
     weight gradients: dW = sum over (t, b) of z_t[b, pre] dpsc_t[b, post]
@@ -239,7 +239,7 @@ class _FusedBPTT(torch.autograd.Function):
             st = _Steps(B, n, C, ctx.has_gk, ctx.has_ref, ctx.proj, ctx.c_in, dev)
         Cb = st.I.shape[0]
         G_psc, G_I = new(Cb, B, n), new(Cb, B, n)  # dL/dpsc_t (state after step t), dL/dI_t of one chunk
-        gz, gT_work = new(B, n), new(B * n)
+        gz, gT_work = new(B, n), new((B + 3) // 4 * 4 * n)
         g_v = [new(B, n), new(B, n)]
         g_gk = [new(B, n), new(B, n)] if ctx.has_gk else None
         g_psc = torch.zeros((B, n), device=dev) if gpT is None else gpT.reshape(B, n).contiguous().clone()
@@ -271,9 +271,9 @@ class _FusedBPTT(torch.autograd.Function):
                     cur_v = gV[t] if cur_v is None else cur_v + gV[t]
                 if gGK is not None and ctx.has_gk:
                     cur_gk = gGK[t] if cur_gk is None else cur_gk + gGK[t]
-                L.check(L.lib().bt_spmv_grad_input_t(B, n, n, lay.csr_ptr.data_ptr(), lay.csr_dst.data_ptr(),
-                                                     w_csr.data_ptr(), gp.data_ptr(), gz.data_ptr(),
-                                                     gT_work.data_ptr(), s), "bt_spmv_grad_input_t")
+                L.check(L.lib().bt_spmv_grad_input_pad(B, n, n, lay.csr_ptr.data_ptr(), lay.csr_dst.data_ptr(),
+                                                       w_csr.data_ptr(), gp.data_ptr(), gz.data_ptr(),
+                                                       gT_work.data_ptr(), s), "bt_spmv_grad_input_pad")
                 if gZ is not None:
                     gz.add_(gZ[t])
                 out_v = g_v[tl & 1]

@@ -159,10 +159,18 @@ BT_API int bt_spmv_grad_input(int64_t batch, int64_t n_in, int64_t n_out,
 
 /* The same product through grad_out transposed into `work` (batch * n_out
  * floats, caller scratch): every edge then reads one contiguous run of
- * samples instead of one scattered word per sample.  Each grad_x[b, j] is
- * an fmaf chain over j's out-edges in CSR order (deterministic; rounding
- * differs from bt_spmv_grad_input's lane-split sum). */
+ * samples instead of one scattered word per sample.  Each grad_x[b, j] is a
+ * fixed tree of fmaf chains over j's out-edges in CSR order (deterministic;
+ * rounding differs from bt_spmv_grad_input's lane-split sum). */
 BT_API int bt_spmv_grad_input_t(int64_t batch, int64_t n_in, int64_t n_out,
+                       const int32_t* csr_ptr, const uint32_t* csr_dst,
+                       const float* csr_w, const float* grad_out,
+                       float* grad_x, float* work, void* stream);
+
+/* bt_spmv_grad_input_t with scratch of 4 * ceil(batch / 4) * n_out floats: the
+ * transposed rows are padded to whole 16-byte runs, so that a batch that is
+ * not a multiple of 4 reads as fast as one that is.  Deterministic. */
+BT_API int bt_spmv_grad_input_pad(int64_t batch, int64_t n_in, int64_t n_out,
                        const int32_t* csr_ptr, const uint32_t* csr_dst,
                        const float* csr_w, const float* grad_out,
                        float* grad_x, float* work, void* stream);
