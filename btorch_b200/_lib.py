@@ -77,6 +77,8 @@ _PROTOS = {
     "bt_spmv_grad_input_t": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bt_spmv_grad_input_pad": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bt_spmv_grad_weight": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "bt_grad_weight_work_words": (C.c_int64, [_i64, _i64, _i32]),
+    "bt_spmv_grad_weight_rows": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _vp, _vp]),
     "bt_check_neuron_desc": (C.c_int, [C.POINTER(BtNeuronDesc)]),
     "bt_fast_div_check": (C.c_int, [C.c_float, C.c_float, _vp, _vp]),
     "bt_neuron_step": (C.c_int, [C.POINTER(BtNeuronDesc), _i64, _i64] + [_vp] * 11 + [_vp]),

@@ -169,10 +169,11 @@ class SparseMM(torch.autograd.Function):
             gw = torch.zeros(0, device=g.device, dtype=torch.float32)
         elif ctx.needs_input_grad[1]:
             gw = torch.empty(layout.nnz, device=g.device, dtype=torch.float32)
-            masks = torch.empty(max(1, n_in * ((B + 31) // 32)), device=g.device, dtype=torch.int32)
-            L.check(L.lib().bt_spmv_grad_weight(B, n_in, layout.n_out, layout.csc_ptr.data_ptr(),
-                                                layout.csc_src.data_ptr(), x.data_ptr(), g.data_ptr(),
-                                                gw.data_ptr(), masks.data_ptr(), s), "bt_spmv_grad_weight")
+            work = torch.empty(L.lib().bt_grad_weight_work_words(B, n_in, 1), device=g.device, dtype=torch.int32)
+            L.check(L.lib().bt_spmv_grad_weight_rows(B, n_in, layout.n_out, layout.csc_ptr.data_ptr(),
+                                                     layout.csc_src.data_ptr(), x.data_ptr(), g.data_ptr(),
+                                                     gw.data_ptr(), 0, 1, work.data_ptr(), s),
+                    "bt_spmv_grad_weight_rows")
         return gx, gw, None, None, None
 
 

@@ -18,7 +18,7 @@ hand-written backward kernels:
                       dI_t, dv_{t-1}, dgk_{t-1} = neuron'(dz_t, dv_t, dgk_t)
                       dpsc_{t-1} = dpsc_t + coef*((-dpsc_t)/tau) + dI_t   (bt_psc_step)
     weight gradients: dW = sum over (t, b) of z_t[b, pre] dpsc_t[b, post]
-                      (bt_spmv_grad_weight, stored nonzeros only);
+                      (bt_spmv_grad_weight_rows, stored nonzeros only);
                       dW_in = sum over (t, b) of x_t[b]^T dI_t[b], over the
                       nonzero inputs only (bt_input_grad_weight).
 
@@ -249,8 +249,8 @@ class _FusedBPTT(torch.autograd.Function):
         want_mag, want_x = ctx.needs_input_grad[3], ctx.needs_input_grad[0]
         want_w, want_b = ctx.proj and ctx.needs_input_grad[1], ctx.proj and ctx.needs_input_grad[2]
         g_mag = torch.empty(lay.nnz, device=dev, dtype=torch.float32) if want_mag else None
-        mag_tmp = torch.empty_like(g_mag) if (want_mag and ctx.n_ch > 1) else None
-        masks = torch.empty(max(1, n * ((Cb * B + 31) // 32)), device=dev, dtype=torch.int32) if want_mag else None
+        mag_work = torch.empty(L.lib().bt_grad_weight_work_words(Cb * B, n, 0), device=dev,
+                               dtype=torch.int32) if want_mag else None
         g_wt = new(ctx.c_in, n) if want_w else None
         gw_work = torch.empty(max(1, ctx.c_in * (Cb * B + 1)), device=dev, dtype=torch.int32) if want_w else None
         g_b = torch.zeros(n, device=dev) if want_b else None
@@ -297,12 +297,10 @@ class _FusedBPTT(torch.autograd.Function):
                 cur_gk = cur_gk.clone()
             rows = kc * B
             if want_mag:
-                dst = g_mag if ci == ctx.n_ch - 1 else mag_tmp
-                L.check(L.lib().bt_spmv_grad_weight(rows, n, n, lay.csc_ptr.data_ptr(), lay.csc_src.data_ptr(),
-                                                    Z[k].data_ptr(), G_psc.data_ptr(), dst.data_ptr(),
-                                                    masks.data_ptr(), s), "bt_spmv_grad_weight")
-                if dst is mag_tmp:
-                    g_mag.add_(mag_tmp)
+                L.check(L.lib().bt_spmv_grad_weight_rows(rows, n, n, lay.csc_ptr.data_ptr(), lay.csc_src.data_ptr(),
+                                                         Z[k].data_ptr(), G_psc.data_ptr(), g_mag.data_ptr(),
+                                                         int(ci != ctx.n_ch - 1), 0, mag_work.data_ptr(), s),
+                        "bt_spmv_grad_weight_rows")
             if want_w:
                 L.check(L.lib().bt_input_grad_weight(rows, ctx.c_in, n, xin[k].data_ptr(), G_I.data_ptr(),
                                                      g_wt.data_ptr(), int(ci != ctx.n_ch - 1), gw_work.data_ptr(),

@@ -185,6 +185,19 @@ BT_API int bt_spmv_grad_weight(int64_t batch, int64_t n_in, int64_t n_out,
                         const float* x, const float* grad_out, float* grad_w,
                         uint32_t* masks, void* stream);
 
+/* The same gradient for many rows (samples, or steps x samples): each source's
+ * nonzero rows are listed once in `work`, then the edges walk the lists over
+ * gradient columns in shared memory.  accumulate != 0 adds to grad_w.
+ * with_dense != 0 (and at most 4096 rows): an x that is mostly nonzero, as
+ * counted on the device, goes through dot products of transposed rows instead
+ * (a fixed tree of fmaf chains).  `work`: bt_grad_weight_work_words(rows, n_in,
+ * with_dense) int32 words, 16-byte aligned. */
+BT_API int64_t bt_grad_weight_work_words(int64_t rows, int64_t n_in, int32_t with_dense);
+BT_API int bt_spmv_grad_weight_rows(int64_t rows, int64_t n_in, int64_t n_out,
+                        const int32_t* csc_ptr, const uint32_t* csc_src,
+                        const float* x, const float* grad_out, float* grad_w,
+                        int32_t accumulate, int32_t with_dense, int32_t* work, void* stream);
+
 /* ------------------------------------------------------------------ */
 /* Neuron and synapse parameter descriptors.                           */
 /* ------------------------------------------------------------------ */
