@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(kGwThreads) k_grad_weight_lists(int64_t r0, in
   int32_t off[kGwPosts + 1];
 #pragma unroll
   for (int p = 0; p <= kGwPosts; ++p) off[p] = csc_ptr[i0 + p < n_out ? i0 + p : n_out];
+  __syncthreads();
   const bool graded = *reinterpret_cast<const volatile int32_t*>(ctl + 2) != 0;
   // the source two edges ahead and the head of the next edge's list are in
   // flight while a list is walked

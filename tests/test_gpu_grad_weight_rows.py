@@ -26,10 +26,9 @@ def grad_weight(lay, x, g, n_in, dense, into=None):
 
 @pytest.mark.parametrize("rows", [1, 6, 7, 8, 15, 16, 31, 33, 64, 130, 4096, 4097, 8200])
 @pytest.mark.parametrize("kind", ["spikes", "graded", "dense"])
-@pytest.mark.parametrize("n_out", [1, 8, 61])
-def test_grad_weight_rows(rows, kind, n_out):
+@pytest.mark.parametrize("n_out,n_in", [(1, 70), (8, 70), (61, 70), (19, 900)])
+def test_grad_weight_rows(rows, kind, n_out, n_in):
     rng = np.random.default_rng(rows * 7 + n_out)
-    n_in = 70
     mask = rng.random((n_out, n_in)) < 0.4
     post, src = np.nonzero(mask)
     m = SparseConn.from_canonical(post, src, np.ones(post.size, np.float32), (n_in, n_out), enforce_dale=False).to(DEV)
