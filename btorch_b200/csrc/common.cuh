@@ -92,6 +92,26 @@ __device__ __forceinline__ float ld_f32(const float* ptr, uint64_t pol) {
 __device__ __forceinline__ void st_f32(float* ptr, float v, uint64_t pol) {
   asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(ptr), "f"(v), "l"(pol) : "memory");
 }
+// 16-byte loads / stores of four consecutive floats with an L2 policy.
+__device__ __forceinline__ float4 ld_nc_f4(const float* ptr, uint64_t pol) {
+  float4 v;
+  asm("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "l"(ptr), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ float4 ld_f4(const float* ptr, uint64_t pol) {
+  float4 v;
+  asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(ptr), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ void st_f4(float* ptr, float4 v, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(ptr), "f"(v.x), "f"(v.y),
+               "f"(v.z), "f"(v.w), "l"(pol)
+               : "memory");
+}
 // fp32 reduction (no return value) with an L2 policy.
 __device__ __forceinline__ void red_add_f32(float* ptr, float v, uint64_t pol) {
   // no "memory" clobber: nothing in the issuing kernel reads the target, so

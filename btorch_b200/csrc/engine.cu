@@ -357,6 +357,160 @@ __global__ void __launch_bounds__(kEngThreads) k_eng_neuron(bt_engine_desc d, in
   publish_spikes_ws(ws, i, b0, spiked);
 }
 
+// Publish the spikes of one sample for the 4 neurons i0 .. i0 + 3 of this
+// thread (bit q of `nib`: neuron i0 + q), as publish_spikes_ws.  The warp's
+// 128 neurons share a sub-list when cap >= 128 (one atomic for the warp),
+// otherwise every lane appends its own.  Called by every lane of the warp.
+__device__ __forceinline__ void publish_nibble(const ScatterScratch& ws, int i0, int b, uint32_t nib) {
+  const unsigned lane = lane_id();
+  uint32_t first = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (nib & (1u << q)) {
+      atomicOr(ws.mask + int64_t(i0 + q) * ws.ms + (b >> 5), 1u << (b & 31));
+      if (atomicOr(ws.flag + i0 + q, 1) == 0) first |= 1u << q;
+    }
+  const int cnt = __popc(first), nspk = __popc(nib);
+  int64_t at;
+  if (ws.cap_shift >= 7) {
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (int(lane) >= o) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const int sub = (i0 - 4 * int(lane)) >> ws.cap_shift;  // the same for the whole warp
+    const int spk = __reduce_add_sync(0xffffffffu, unsigned(nspk));
+    int base = 0;
+    if (lane == 0) {
+      atomicAdd(ws.spk + sub, spk);
+      if (total) base = atomicAdd(ws.count + sub, total);
+    }
+    base = __shfl_sync(0xffffffffu, base, 0);
+    at = int64_t(sub) * ws.cap + base + incl - cnt;
+  } else {
+    const int sub = i0 >> ws.cap_shift;
+    if (nspk) atomicAdd(ws.spk + sub, nspk);
+    at = int64_t(sub) * ws.cap + (cnt ? atomicAdd(ws.count + sub, cnt) : 0);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (first & (1u << q)) ws.list[at++] = i0 + q;
+}
+
+// The same step for n a multiple of 4 and 16-byte aligned arrays: a thread
+// owns 4 consecutive neurons of one sample, so every array moves in 16-byte
+// accesses (6 in flight per thread, all before the first store) and the
+// bookkeeping -- sample length, addresses, bitmap words, publication -- is paid
+// once per 4 neurons instead of once per neuron-sample, which is what the
+// per-neuron kernel's time went to (its issue slots, 71 %).  A block of a
+// finished sample only writes its zero words.  A warp covers 4 bitmap words;
+// publication runs only in warps with a spike.  Grid (ceil(n / 512), batch),
+// 128 threads.  z_given: publish these spikes instead of the step's own (a
+// recomputation driven by the spikes of its first run).
+constexpr int kVecThreads = 128;
+template <int KIND, bool HARD, bool USE_REF, bool FAST>
+__global__ void __launch_bounds__(kVecThreads) k_eng_neuron_vec(bt_engine_desc d, int k, StepIdx si, ScatterScratch ws,
+                                                                const float* __restrict__ z_given) {
+  const int n = int(d.n), B = int(d.batch);
+  const int words = (n + 31) >> 5;
+  const int i0 = (int(blockIdx.x) * kVecThreads + int(threadIdx.x)) * 4;
+  const int b = int(blockIdx.y);
+  const unsigned lane = lane_id();
+  if (i0 - 4 * int(lane) >= n) return;  // whole warps past the end
+  const bool valid = i0 < n;            // n % 4 == 0: all four or none
+  const int len = d.sample_len ? d.sample_len[b] : INT_MAX;
+  const bool st_traces = d.v_trace || d.psc_trace || d.ref_trace || d.gk_trace;
+  uint32_t* hist_p = d.hist + (int64_t(si.h_t) * B + b) * words + (i0 >> 5);
+  uint32_t* raster_p = d.raster ? d.raster + (int64_t(k) * B + b) * words + (i0 >> 5) : nullptr;
+  if (k > len && !st_traces && !d.spikes) {  // block-uniform: frozen, nothing to read
+    if (valid && (lane & 7) == 0) {
+      *hist_p = 0u;
+      if (raster_p) *raster_p = 0u;
+    }
+    return;
+  }
+  const int o = b * n + (valid ? i0 : 0);
+  const int64_t tix = int64_t(k) * B * n + o;
+  const uint64_t pol_stream = l2_evict_first(), pol_keep = l2_evict_last();
+  const bool live = k < len, edge = k <= len;
+  const bool want = valid && (edge || st_traces);
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 aq = zero, pq = zero, xq = zero, vq = zero, rq = zero, gq = zero, zq = zero;
+  if (want) {
+    if (edge) aq = ld_f4(d.ring + o, pol_keep);
+    pq = *reinterpret_cast<const float4*>(d.psc + o);
+    if (live && d.x) xq = ld_nc_f4(d.x + tix, pol_stream);
+    vq = *reinterpret_cast<const float4*>(d.v + o);
+    if (USE_REF) rq = *reinterpret_cast<const float4*>(d.refractory + o);
+    if (KIND == BT_NEURON_ALIF) gq = *reinterpret_cast<const float4*>(d.g_k + o);
+    if (z_given) zq = ld_nc_f4(z_given + tix, pol_stream);
+  }
+  float acc[4] = {aq.x, aq.y, aq.z, aq.w}, P[4] = {pq.x, pq.y, pq.z, pq.w}, x[4] = {xq.x, xq.y, xq.z, xq.w};
+  float v[4] = {vq.x, vq.y, vq.z, vq.w}, ref[4] = {rq.x, rq.y, rq.z, rq.w}, gk[4] = {gq.x, gq.y, gq.z, gq.w};
+  float s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, stored[4];
+  NeuronParams prm = load_params<KIND, USE_REF>(d.neuron, valid ? i0 : 0);
+  float pc = d.psc_uniform ? d.psc_coef_s : 0.0f;
+  Div dpt = make_div(d.psc_uniform ? d.psc_tau_s : 1.0f, d.psc_uniform && d.psc_fast_div, d.psc_rcp);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = valid ? i0 + q : 0;
+    if (!FAST) {  // (FAST: every parameter a scalar)
+      if (q > 0 && !d.neuron.uniform) prm = load_params<KIND, USE_REF>(d.neuron, i);
+      if (!d.psc_uniform) {
+        pc = ld(d.psc_coef, i);
+        dpt = make_div(ld(d.psc_tau, i), false, 0.0f);
+      }
+    }
+    if (edge) P[q] = add(P[q], acc[q]);
+    stored[q] = P[q];
+    if (live) {
+      const float I = d.x ? add(P[q], x[q]) : P[q];
+      s[q] = neuron_update<KIND, HARD, USE_REF, true, FAST>(prm, I, v[q], ref[q], gk[q]).spike;
+      stored[q] = psc_decay_k<FAST>(pc, dpt, P[q]);
+    }
+  }
+  uint32_t nib = 0, own = 0;
+  if (valid) {
+    if (edge) {
+      st_f4(d.ring + o, zero, pol_keep);
+      *reinterpret_cast<float4*>(d.psc + o) = make_float4(stored[0], stored[1], stored[2], stored[3]);
+    }
+    if (live) {
+      *reinterpret_cast<float4*>(d.v + o) = make_float4(v[0], v[1], v[2], v[3]);
+      if (USE_REF) *reinterpret_cast<float4*>(d.refractory + o) = make_float4(ref[0], ref[1], ref[2], ref[3]);
+      if (KIND == BT_NEURON_ALIF) *reinterpret_cast<float4*>(d.g_k + o) = make_float4(gk[0], gk[1], gk[2], gk[3]);
+    }
+    if (st_traces) {
+      auto put = [&](float* t, int64_t at, const float(&q)[4]) {
+        if (t) *reinterpret_cast<float4*>(t + at) = make_float4(q[0], q[1], q[2], q[3]);
+      };
+      if (k > 0) put(d.psc_trace, tix - int64_t(B) * n, P);
+      put(d.v_trace, tix, v);
+      if (USE_REF) put(d.ref_trace, tix, ref);
+      if (KIND == BT_NEURON_ALIF) put(d.gk_trace, tix, gk);
+    }
+    if (d.spikes) *reinterpret_cast<float4*>(d.spikes + tix) = make_float4(s[0], s[1], s[2], s[3]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) own |= (s[q] != 0.0f ? 1u : 0u) << q;
+    nib = own;
+    if (z_given)
+      nib = (zq.x != 0.0f ? 1u : 0u) | (zq.y != 0.0f ? 2u : 0u) | (zq.z != 0.0f ? 4u : 0u) | (zq.w != 0.0f ? 8u : 0u);
+  }
+  const bool any = __any_sync(0xffffffffu, nib != 0);
+  uint32_t word = nib << (4 * (lane & 7));
+  if (any) {  // the word of the 8 lanes' 32 neurons
+#pragma unroll
+    for (int w = 1; w < 8; w <<= 1) word |= __shfl_xor_sync(0xffffffffu, word, w);
+  }
+  if (valid && (lane & 7) == 0) {
+    *hist_p = word;
+    if (raster_p) *raster_p = word;
+  }
+  if (any) publish_nibble(ws, i0, b, nib);
+}
+
 // SCATTER neuron step with receptor channels (n_rec = C > 1): for each
 // channel column c = i * C + r, P_r = stored + acc (acc zeroed); the neuron's
 // input is receptor_sum(P) (+ x); stored = decay_r(P_r).  Grid
@@ -1548,7 +1702,7 @@ bool fast_divisors(const bt_engine_desc& d, int kind) {
 }
 
 template <int KIND, bool HARD, bool USE_REF>
-int run_typed(const bt_engine_desc& d, cudaStream_t s) {
+int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
   const int64_t n = d.n;
   if (d.mode == BT_MODE_CLUSTER) return run_cluster(d, fast_divisors(d, KIND), s);  // no final launch
   if (d.mode == BT_MODE_TILE) {
@@ -1591,6 +1745,17 @@ int run_typed(const bt_engine_desc& d, cudaStream_t s) {
     const dim3 rgrid(unsigned(ceil_div(n, kEngThreads)), unsigned(d.batch));
     // vector access to the C channels of (b, i) needs 8 / 16-byte aligned state and acc
     const bool aligned = ((reinterpret_cast<uintptr_t>(d.psc) | reinterpret_cast<uintptr_t>(d.ring)) & 15) == 0;
+// The arrays the scatter neuron step touches admit 16-byte accesses.
+bool vec_neurons(const bt_engine_desc& d, const float* z_given) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(d.v) | reinterpret_cast<uintptr_t>(d.psc) |
+                      reinterpret_cast<uintptr_t>(d.refractory) | reinterpret_cast<uintptr_t>(d.g_k) |
+                      reinterpret_cast<uintptr_t>(d.ring) | reinterpret_cast<uintptr_t>(d.x) |
+                      reinterpret_cast<uintptr_t>(d.spikes) | reinterpret_cast<uintptr_t>(d.v_trace) |
+                      reinterpret_cast<uintptr_t>(d.psc_trace) | reinterpret_cast<uintptr_t>(d.ref_trace) |
+                      reinterpret_cast<uintptr_t>(d.gk_trace) | reinterpret_cast<uintptr_t>(z_given);
+  return d.n % 4 == 0 && (a & 15) == 0 && d.batch < 65536;
+}
+
     auto rec = C == 4 && aligned ? k_eng_neuron_rec<KIND, HARD, USE_REF, 4>
              : C == 2 && aligned ? k_eng_neuron_rec<KIND, HARD, USE_REF, 2> : k_eng_neuron_rec<KIND, HARD, USE_REF, 0>;
     for (int64_t k = 0; k < d.n_steps; ++k) {
@@ -1636,9 +1801,13 @@ int run_typed(const bt_engine_desc& d, cudaStream_t s) {
       else BT_PULL_LAUNCH(4);
     }
 #undef BT_PULL_LAUNCH
+    const bool vec = C == 1 && vec_neurons(d, z_given);
+    const dim3 vgrid(unsigned(ceil_div(n, 4 * kVecThreads)), unsigned(d.batch));
+    auto nvec = fast ? k_eng_neuron_vec<KIND, HARD, USE_REF, true> : k_eng_neuron_vec<KIND, HARD, USE_REF, false>;
   } else {
     const int grid = int(ceil_div(n, 32));
     const size_t smem = sizeof(uint32_t) * size_t(d.batch);
+      else if (vec) nvec<<<vgrid, kVecThreads, 0, s>>>(d, int(k), si, scatter_scratch(d, si.q_t), z_given);
     BT_CHECK_ARG(smem <= 48 * 1024, "batch too large for the gather engine");
     auto gather = n_rec(d) > 1 ? k_eng_gather<KIND, HARD, USE_REF, true> : k_eng_gather<KIND, HARD, USE_REF, false>;
     for (int64_t k = 0; k < d.n_steps; ++k)
@@ -1654,7 +1823,8 @@ int run_typed(const bt_engine_desc& d, cudaStream_t s) {
 
 }  // namespace
 
-extern "C" int bt_engine_run(const bt_engine_desc* d, void* stream) {
+namespace {
+int engine_run(const bt_engine_desc* d, const float* z_given, void* stream) {
   if (int st = engine_check(d)) return st;
   if (d->n_steps == 0) return BT_OK;
   if (d->stats && cudaMemsetAsync(d->stats, 0, sizeof(int64_t) * 4 * size_t(d->n_steps),
@@ -1663,15 +1833,15 @@ extern "C" int bt_engine_run(const bt_engine_desc* d, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool h = d->neuron.hard_reset != 0, r = d->neuron.use_refractory != 0;
   if (d->neuron.kind == BT_NEURON_LIF) {
-    if (h && r) return run_typed<BT_NEURON_LIF, true, true>(*d, s);
-    if (h) return run_typed<BT_NEURON_LIF, true, false>(*d, s);
-    if (r) return run_typed<BT_NEURON_LIF, false, true>(*d, s);
-    return run_typed<BT_NEURON_LIF, false, false>(*d, s);
+    if (h && r) return run_typed<BT_NEURON_LIF, true, true>(*d, z_given, s);
+    if (h) return run_typed<BT_NEURON_LIF, true, false>(*d, z_given, s);
+    if (r) return run_typed<BT_NEURON_LIF, false, true>(*d, z_given, s);
+    return run_typed<BT_NEURON_LIF, false, false>(*d, z_given, s);
   }
-  if (h && r) return run_typed<BT_NEURON_ALIF, true, true>(*d, s);
-  if (h) return run_typed<BT_NEURON_ALIF, true, false>(*d, s);
-  if (r) return run_typed<BT_NEURON_ALIF, false, true>(*d, s);
-  return run_typed<BT_NEURON_ALIF, false, false>(*d, s);
+  if (h && r) return run_typed<BT_NEURON_ALIF, true, true>(*d, z_given, s);
+  if (h) return run_typed<BT_NEURON_ALIF, true, false>(*d, z_given, s);
+  if (r) return run_typed<BT_NEURON_ALIF, false, true>(*d, z_given, s);
+  return run_typed<BT_NEURON_ALIF, false, false>(*d, z_given, s);
 }
 
 extern "C" int bt_engine_prime(const bt_engine_desc* d, void* stream) {
@@ -1716,6 +1886,9 @@ extern "C" int bt_input_project(int64_t rows, int64_t c_in, int64_t n, const flo
                                 const float* bias, float* out, int32_t* work, void* stream) {
   return input_project(rows, c_in, n, xin, w_t, bias, out, work, nullptr, 1, stream);
 }
+}  // namespace
+
+extern "C" int bt_engine_run(const bt_engine_desc* d, void* stream) { return engine_run(d, nullptr, stream); }
 
 extern "C" int bt_input_project_live(int64_t steps, int64_t batch, int64_t c_in, int64_t n, const float* xin,
                                      const float* w_t, const float* bias, const int32_t* sample_len, float* out,

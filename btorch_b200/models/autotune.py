@@ -119,7 +119,9 @@ def candidates(conn, batch: int, receptors: int = 1, n_bins: int = 1, n: int = 0
                     out.append(EngineChoice(mode, tile_posts=0 if mult == 1 else tp))
             continue
         if mode == L.BT_MODE_SCATTER:
-            for spt in (1, 2, 4):
+            # (n a multiple of 4 without receptor channels: the vectorised neuron
+            # step, whatever spt)
+            for spt in (1, 2, 4) if n % 4 or receptors > 1 or n == 0 else (1,):
                 if spt > 1 and spt > batch:
                     continue
                 for lanes in (1, 8, 32):
