@@ -632,37 +632,90 @@ __global__ void __launch_bounds__(kEngThreads) k_eng_neuron_rec(bt_engine_desc d
   publish_spikes<1>(d, si, i, b, s != 0.0f ? 1u : 0u);
 }
 
-// Offsets of the kSub sub-lists of one spike set in shared memory (warp 0
-// scans the counts; two per lane).
-__device__ __forceinline__ void sub_offsets(const ScatterScratch& ws, int32_t* s_off, int32_t* s_spk) {
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-    const int32_t c0 = ws.count[2 * l], c1 = ws.count[2 * l + 1];
-    int32_t v = c0 + c1;
-    int32_t sp = ws.spk[2 * l] + ws.spk[2 * l + 1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int32_t y = __shfl_up_sync(0xffffffffu, v, o);
-      if (l >= o) v += y;
-      sp += __shfl_xor_sync(0xffffffffu, sp, o);
-    }
-    s_off[2 * l] = v - c0 - c1;
-    s_off[2 * l + 1] = v - c1;
-    if (l == 31) s_off[kSub] = v;
-    if (l == 0) *s_spk = sp;
+// Offsets of the sub-lists of every delivered spike set (planes x kSub, plane y
+// = delay bin bin_lo + y, the set of step t - bin) in shared memory: s_off[c] =
+// rows listed before counter c, s_off[planes * kSub] = rows of the step.  One
+// list over all planes lets every warp of the grid take its share of the rows
+// whatever bin they belong to.  *s_spk: spikes listed (one plane only).
+__device__ __forceinline__ void plane_offsets(const bt_engine_desc& d, const StepIdx& si, int planes, int32_t* s_off,
+                                              int32_t* s_spk) {
+  __shared__ int32_t s_warp[kEngThreads / 32];
+  const int Q = d.n_bins + 1, total = planes * kSub;
+  const int per = (total + kEngThreads - 1) / kEngThreads;
+  const int c0 = int(threadIdx.x) * per, c1 = c0 + per < total ? c0 + per : total;
+  int32_t sum = 0, spk = 0;
+#pragma unroll 4
+  for (int c = c0; c < c1; ++c) {
+    int q = si.q_t - d.bin_lo - c / kSub;
+    if (q < 0) q += Q;
+    const int32_t* cnt = d.work + q * 2 * kSub + c % kSub;
+    const int32_t v = cnt[0];
+    if (planes == 1) spk += cnt[kSub];
+    s_off[c] = v;
+    sum += v;
   }
+  const int lane = int(lane_id()), warp = int(threadIdx.x >> 5);
+  int32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  if (threadIdx.x == 0) *s_spk = 0;
+  __syncthreads();
+  if (planes == 1 && spk) atomicAdd(s_spk, spk);
+  int32_t run = incl - sum;
+#pragma unroll
+  for (int w = 0; w < kEngThreads / 32; ++w) run += w < warp ? s_warp[w] : 0;
+  for (int c = c0; c < c1; ++c) {
+    const int32_t v = s_off[c];
+    s_off[c] = run;
+    run += v;
+  }
+  if (threadIdx.x == kEngThreads - 1) s_off[total] = run;
   __syncthreads();
 }
 
-// Sub-list holding item `it`: the last s with s_off[s] <= it (s_off[kSub] > it).
-__device__ __forceinline__ int find_sub(const int32_t* s_off, int64_t it) {
-  int lo = 0, hi = kSub - 1;
+// Counter holding item `it`: the last c with s_off[c] <= it (s_off[total] > it).
+__device__ __forceinline__ int find_sub(const int32_t* s_off, int total, int32_t it) {
+  int lo = 0, hi = total - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (s_off[mid] <= it) lo = mid;
     else hi = mid - 1;
   }
   return lo;
+}
+
+// One listed row of the step: its neuron, delay bin and sample mask.
+struct ListedRow {
+  int32_t j;
+  int bin;
+  uint32_t* mask;
+  int32_t* flag;
+};
+
+__device__ __forceinline__ ListedRow listed_row(const bt_engine_desc& d, const StepIdx& si, const ScatterScratch& ws0,
+                                                const int32_t* s_off, int planes, int32_t it) {
+  const int c = find_sub(s_off, planes * kSub, it);
+  ListedRow r;
+  r.bin = d.bin_lo + c / kSub;
+  int q = si.q_t - r.bin;
+  if (q < 0) q += d.n_bins + 1;
+  r.j = ws0.list[(int64_t(q) * kSub + c % kSub) * ws0.cap + (it - s_off[c])];
+  r.mask = ws0.mask + (int64_t(q) * d.n + r.j) * ws0.ms;
+  r.flag = ws0.flag + int64_t(q) * d.n + r.j;
+  return r;
+}
+
+// The counts of slot (t + 1) mod Q, i.e. of step t - R, were last read by the
+// previous step's scatter: clear them for the next neuron launch.
+__device__ __forceinline__ void clear_oldest_counts(const bt_engine_desc& d, const StepIdx& si) {
+  if (blockIdx.x == 0 && threadIdx.x < 2 * kSub) {
+    const int qc = si.q_t + 1 == d.n_bins + 1 ? 0 : si.q_t + 1;
+    d.work[qc * 2 * kSub + threadIdx.x] = 0;
+  }
 }
 
 // Block-level sum of per-thread event / edge counts, one pair of atomics per
@@ -713,8 +766,7 @@ __device__ void scatter_dense(const bt_engine_desc& d, int64_t k, const ScatterS
   const int64_t nc = n * n_rec(d);  // acc columns (post * C + r)
   const int n32 = int(nc);
   const int64_t n_slices = (nc + 31) >> 5;
-  const int64_t nblocks = int64_t(gridDim.x) * gridDim.y;
-  const int64_t bid = int64_t(blockIdx.y) * gridDim.x + blockIdx.x;
+  const int64_t nblocks = gridDim.x, bid = blockIdx.x;
   float(*acc)[32] = s_acc[wid];
   const uint64_t pol_stream = l2_evict_first();
   const uint32_t sentinel = uint32_t(n);
@@ -783,44 +835,40 @@ __device__ void scatter_dense(const bt_engine_desc& d, int64_t k, const ScatterS
   }
 }
 
-// Grid (x, bin_hi - bin_lo + 1): plane y delivers delay bin d = bin_lo + y,
-// i.e. the spike set of step t - d through rows j * R + d.  G lanes share one
-// row (G = 32 for long rows, 8 for the short rows of a wide delay range), each
-// lane loading 4 edges with one 128-bit load of posts and one of weights, then
-// adding them for every sample in the row's mask (MS words; the sample loop is
-// outside the edge loop, so a lane issues 4 reductions per mask bit).
+// Delivery of one step: for every listed neuron j of the spike set of step
+// t - bin, for every delay bin, row j * R + bin.  G lanes share one row, each
+// lane loading 4 edges with two 128-bit loads of records, then adding them for
+// every sample in the row's mask (MS words; the sample loop is outside the edge
+// loop, so a lane issues 4 reductions per mask bit).  The grid is one wave of
+// resident blocks over the rows of all bins: a step is a
+// chain of dependent loads per row (list, row pointers and mask, edges), so a
+// second wave, or planes of a bin each with idle warps beside busy ones, costs
+// the whole chain again (20 bins, 120k rows of 6 edges: 12.9 us a step with a
+// plane of blocks per bin and two waves).
 // Launch bounds: at least 4 (MS <= 4) or 3 resident blocks per SM, which
 // leaves ptxas 64 / 85 registers -- without a bound its occupancy heuristic
 // has settled on 48 registers and spilled the reduction loop.
 template <int G, int MS>
 __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt_engine_desc d, int64_t k, StepIdx si) {
+  extern __shared__ int32_t s_off[];  // [planes * kSub + 1]
   const int64_t n = d.n;
-  const int R = d.n_bins, Q = R + 1;
-  const int bin = d.bin_lo + int(blockIdx.y);
-  int q = si.q_t - bin;
-  if (q < 0) q += Q;
-  const ScatterScratch ws = scatter_scratch(d, q);
-  __shared__ int32_t s_off[kSub + 1];
+  const int R = d.n_bins, planes = d.bin_hi - d.bin_lo + 1;
+  const ScatterScratch ws0 = scatter_scratch(d, 0);
   __shared__ int32_t s_spk;
-  sub_offsets(ws, s_off, &s_spk);
-  const int32_t count = s_off[kSub];
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kSub) {
-    // the counts of slot (t + 1) mod Q, i.e. of step t - R, were last read by
-    // the previous step's scatter: clear them for the next neuron launch
-    const int qc = si.q_t + 1 == Q ? 0 : si.q_t + 1;
-    d.work[qc * 2 * kSub + threadIdx.x] = 0;
-    d.work[qc * 2 * kSub + kSub + threadIdx.x] = 0;
-  }
+  plane_offsets(d, si, planes, s_off, &s_spk);
+  const int32_t count = s_off[planes * kSub];
+  clear_oldest_counts(d, si);
   if (blockIdx.x == 0 && threadIdx.x == 0 && d.stats)
     atomicAdd(reinterpret_cast<unsigned long long*>(d.stats + k * 4 + 0), (unsigned long long)count);
   // dense when most neurons spike and they do so in several samples each
   if (d.dense_rows > 0 && count >= d.dense_rows && s_spk >= kDenseSpikesPerRow * count) {  // grid-uniform
+    int q = si.q_t - d.bin_lo;
+    if (q < 0) q += R + 1;
     long long ev = 0, ed = 0;
-    scatter_dense<MS>(d, k, ws, ev, ed);
+    scatter_dense<MS>(d, k, scatter_scratch(d, q), ev, ed);
     if (d.stats) block_stats(d, k, ev, ed);
     return;
   }
-  const bool last_use = bin == d.bin_hi;  // this set is not read again: clear it
   const unsigned lane = lane_id();
   const int grp = int(lane) / G, lig = int(lane) % G;
   constexpr int kPerWarp = 32 / G;
@@ -834,29 +882,29 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
     uint32_t mw_local[MS];
     int32_t beg = 0, end = 0;
     uint32_t* mrow = nullptr;
-    int32_t j = -1;
+    int32_t* flag = nullptr;
     if (it < count) {
-      const int sub = find_sub(s_off, it);
-      j = ws.list[sub * ws.cap + (it - s_off[sub])];
-      mrow = ws.mask + int64_t(j) * ws.ms;
-      const int64_t row = int64_t(j) * R + bin;
+      const ListedRow r = listed_row(d, si, ws0, s_off, planes, int32_t(it));
+      mrow = r.mask;
+      flag = r.bin == d.bin_hi ? r.flag : nullptr;  // this set is not read again: clear it
+      const int64_t row = int64_t(r.j) * R + r.bin;
       beg = d.csr_ptr[row];
       end = d.csr_ptr[row + 1];
     }
-    // MS is the compile-time bound (1, 2, 4 or 8); the row holds ws.ms words
+    // MS is the compile-time bound (1, 2, 4 or 8); the row holds ms words
     // (5..8 samples words above 128 samples run with MS = 8)
     int nsamp = 0;
 #pragma unroll
     for (int w = 0; w < MS; ++w) {
-      mw_local[w] = (mrow && w < ws.ms) ? mrow[w] : 0u;
+      mw_local[w] = (mrow && w < ws0.ms) ? mrow[w] : 0u;
       nsamp += __popc(mw_local[w]);
     }
     __syncwarp();
-    if (last_use && lig == 0 && j >= 0) {
+    if (flag && lig == 0) {
 #pragma unroll
       for (int w = 0; w < MS; ++w)
-        if (w < ws.ms) mrow[w] = 0;
-      ws.flag[j] = 0;
+        if (w < ws0.ms) mrow[w] = 0;
+      *flag = 0;
     }
     if (lig == 0) {
       ev += (long long)nsamp * (end - beg);
@@ -909,66 +957,62 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
 }
 
 // Scatter for short rows (a wide delay range splits each neuron's out-edges
-// into n_bins rows): a warp takes 32 rows, one per lane, scans their lengths
-// and walks their edges as one flattened range, 32 consecutive edges per
-// iteration -- each lane finds its row by a 5-step binary search over the
-// lanes' exclusive offsets (shuffles), so no lane idles on a short row and
-// consecutive lanes load consecutive edges.  Grid as k_eng_scatter.
+// into n_bins rows): a warp takes up to 32 rows -- the step's rows spread evenly
+// over the grid's warps -- one per lane, scans their lengths and walks their
+// edges as one flattened range, 32 consecutive edges per iteration: each lane
+// finds its row by a 5-step binary search over the lanes' exclusive offsets
+// (shuffles), so no lane idles on a short row and consecutive lanes load
+// consecutive edges.  Grid as k_eng_scatter.
 template <int MS>
 __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_flat(bt_engine_desc d, int64_t k,
                                                                               StepIdx si) {
-  const int R = d.n_bins, Q = R + 1;
-  const int bin = d.bin_lo + int(blockIdx.y);
-  int q = si.q_t - bin;
-  if (q < 0) q += Q;
-  const ScatterScratch ws = scatter_scratch(d, q);
-  __shared__ int32_t s_off[kSub + 1];
+  extern __shared__ int32_t s_off[];  // [planes * kSub + 1]
+  const int R = d.n_bins, planes = d.bin_hi - d.bin_lo + 1;
+  const ScatterScratch ws0 = scatter_scratch(d, 0);
   __shared__ int32_t s_spk;
-  sub_offsets(ws, s_off, &s_spk);
-  const int32_t count = s_off[kSub];
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kSub) {
-    const int qc = si.q_t + 1 == Q ? 0 : si.q_t + 1;  // step t - R: last read by the previous step
-    d.work[qc * 2 * kSub + threadIdx.x] = 0;
-    d.work[qc * 2 * kSub + kSub + threadIdx.x] = 0;
-  }
+  plane_offsets(d, si, planes, s_off, &s_spk);
+  const int32_t count = s_off[planes * kSub];
+  clear_oldest_counts(d, si);
   if (blockIdx.x == 0 && threadIdx.x == 0 && d.stats)
     atomicAdd(reinterpret_cast<unsigned long long*>(d.stats + k * 4 + 0), (unsigned long long)count);
   // dense when most neurons spike and they do so in several samples each
   if (d.dense_rows > 0 && count >= d.dense_rows && s_spk >= kDenseSpikesPerRow * count) {  // grid-uniform
+    int q = si.q_t - d.bin_lo;
+    if (q < 0) q += R + 1;
     long long ev = 0, ed = 0;
-    scatter_dense<MS>(d, k, ws, ev, ed);
+    scatter_dense<MS>(d, k, scatter_scratch(d, q), ev, ed);
     if (d.stats) block_stats(d, k, ev, ed);
     return;
   }
-  const bool last_use = bin == d.bin_hi;
   const int lane = int(lane_id());
   const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   const int n32 = int(d.n * n_rec(d));  // acc row stride; batch * n * C < 2^31 (checked on the host)
   const uint64_t pol_stream = l2_evict_first(), pol_keep = l2_evict_last();
   long long ev = 0, ed = 0;
-  for (int64_t base = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * 32; base < count;
-       base += warps * 32) {
+  // rows per warp and pass: an even share of the step's rows, 32 at most
+  const int64_t share = (count + warps - 1) / warps;
+  const int rpw = int(share < 32 ? share : 32);
+  for (int64_t base = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * rpw; base < count;
+       base += warps * rpw) {
     const int64_t it = base + lane;
     uint32_t mw[MS];
     int32_t beg = 0, len = 0;
-    if (it < count) {
-      const int sub = find_sub(s_off, it);
-      const int32_t j = ws.list[sub * ws.cap + (it - s_off[sub])];
-      uint32_t* mrow = ws.mask + int64_t(j) * ws.ms;
-      const int64_t row = int64_t(j) * R + bin;
+    if (lane < rpw && it < count) {
+      const ListedRow r = listed_row(d, si, ws0, s_off, planes, int32_t(it));
+      const int64_t row = int64_t(r.j) * R + r.bin;
       beg = d.csr_ptr[row];
       len = d.csr_ptr[row + 1] - beg;
       int nsamp = 0;
 #pragma unroll
       for (int w = 0; w < MS; ++w) {
-        mw[w] = w < ws.ms ? mrow[w] : 0u;
+        mw[w] = w < ws0.ms ? r.mask[w] : 0u;
         nsamp += __popc(mw[w]);
       }
-      if (last_use) {
+      if (r.bin == d.bin_hi) {  // this set is not read again: clear it
 #pragma unroll
         for (int w = 0; w < MS; ++w)
-          if (w < ws.ms) mrow[w] = 0;
-        ws.flag[j] = 0;
+          if (w < ws0.ms) r.mask[w] = 0;
+        *r.flag = 0;
       }
       ev += (long long)nsamp * len;
       ed += len;
@@ -1701,6 +1745,17 @@ bool fast_divisors(const bt_engine_desc& d, int kind) {
   return ok;
 }
 
+// The arrays the scatter neuron step touches admit 16-byte accesses.
+bool vec_neurons(const bt_engine_desc& d, const float* z_given) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(d.v) | reinterpret_cast<uintptr_t>(d.psc) |
+                      reinterpret_cast<uintptr_t>(d.refractory) | reinterpret_cast<uintptr_t>(d.g_k) |
+                      reinterpret_cast<uintptr_t>(d.ring) | reinterpret_cast<uintptr_t>(d.x) |
+                      reinterpret_cast<uintptr_t>(d.spikes) | reinterpret_cast<uintptr_t>(d.v_trace) |
+                      reinterpret_cast<uintptr_t>(d.psc_trace) | reinterpret_cast<uintptr_t>(d.ref_trace) |
+                      reinterpret_cast<uintptr_t>(d.gk_trace) | reinterpret_cast<uintptr_t>(z_given);
+  return d.n % 4 == 0 && (a & 15) == 0 && d.batch < 65536;
+}
+
 template <int KIND, bool HARD, bool USE_REF>
 int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
   const int64_t n = d.n;
@@ -1717,14 +1772,13 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned planes = unsigned(d.bin_hi - d.bin_lo + 1);
-    // a plane lists at most n rows: no more blocks than n rows need (small
-    // networks would otherwise launch mostly idle blocks every step)
-    const int64_t rows_per_block = d.scatter_lanes == 1 ? kEngThreads : d.scatter_lanes == 8 ? kEngThreads / 8
-                                                                                            : kEngThreads / 32;
-    const int64_t xblocks = std::min(ceil_div(int64_t(sms) * 8, planes), ceil_div(n, rows_per_block));
-    const dim3 sgrid(unsigned(std::max<int64_t>(xblocks, 1)), planes);
+    const int planes = d.bin_hi - d.bin_lo + 1;
     const int ms = mask_stride(d.batch);
+    // one wave of resident blocks, fewer when the step cannot list that many rows
+    const int64_t rows_per_block = d.scatter_lanes == 1 ? 64 : d.scatter_lanes == 8 ? kEngThreads / 8 : kEngThreads / 32;
+    const int64_t wave = int64_t(sms) * (ms <= 4 ? 4 : 3);
+    const unsigned sgrid = unsigned(std::max<int64_t>(1, std::min(wave, ceil_div(n * planes, rows_per_block))));
+    const size_t ssmem = sizeof(int32_t) * size_t(planes * kSub + 1);
     // every divisor a power of two or a verified reciprocal: no IEEE division compiled in
     const bool fast = fast_divisors(d, KIND);
     auto neuron = fast ? (S == 1 ? k_eng_neuron<KIND, HARD, USE_REF, 1, true>
@@ -1745,24 +1799,17 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
     const dim3 rgrid(unsigned(ceil_div(n, kEngThreads)), unsigned(d.batch));
     // vector access to the C channels of (b, i) needs 8 / 16-byte aligned state and acc
     const bool aligned = ((reinterpret_cast<uintptr_t>(d.psc) | reinterpret_cast<uintptr_t>(d.ring)) & 15) == 0;
-// The arrays the scatter neuron step touches admit 16-byte accesses.
-bool vec_neurons(const bt_engine_desc& d, const float* z_given) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(d.v) | reinterpret_cast<uintptr_t>(d.psc) |
-                      reinterpret_cast<uintptr_t>(d.refractory) | reinterpret_cast<uintptr_t>(d.g_k) |
-                      reinterpret_cast<uintptr_t>(d.ring) | reinterpret_cast<uintptr_t>(d.x) |
-                      reinterpret_cast<uintptr_t>(d.spikes) | reinterpret_cast<uintptr_t>(d.v_trace) |
-                      reinterpret_cast<uintptr_t>(d.psc_trace) | reinterpret_cast<uintptr_t>(d.ref_trace) |
-                      reinterpret_cast<uintptr_t>(d.gk_trace) | reinterpret_cast<uintptr_t>(z_given);
-  return d.n % 4 == 0 && (a & 15) == 0 && d.batch < 65536;
-}
-
     auto rec = C == 4 && aligned ? k_eng_neuron_rec<KIND, HARD, USE_REF, 4>
              : C == 2 && aligned ? k_eng_neuron_rec<KIND, HARD, USE_REF, 2> : k_eng_neuron_rec<KIND, HARD, USE_REF, 0>;
+    const bool vec = C == 1 && vec_neurons(d, z_given);
+    const dim3 vgrid(unsigned(ceil_div(n, 4 * kVecThreads)), unsigned(d.batch));
+    auto nvec = fast ? k_eng_neuron_vec<KIND, HARD, USE_REF, true> : k_eng_neuron_vec<KIND, HARD, USE_REF, false>;
     for (int64_t k = 0; k < d.n_steps; ++k) {
       const StepIdx si = step_idx(d.t0 + k, d.n_bins, d.hist_len);
       if (C > 1) rec<<<rgrid, kEngThreads, 0, s>>>(d, k, si);
+      else if (vec) nvec<<<vgrid, kVecThreads, 0, s>>>(d, int(k), si, scatter_scratch(d, si.q_t), z_given);
       else neuron<<<grid, kEngThreads, 0, s>>>(d, int(k), si, scatter_scratch(d, si.q_t));
-      scatter<<<sgrid, kEngThreads, 0, s>>>(d, k, si);
+      scatter<<<sgrid, kEngThreads, ssmem, s>>>(d, k, si);
     }
     BT_CHECK_LAUNCH("k_eng_neuron/k_eng_scatter");
     if (d.n_steps > 0) {
@@ -1801,13 +1848,9 @@ bool vec_neurons(const bt_engine_desc& d, const float* z_given) {
       else BT_PULL_LAUNCH(4);
     }
 #undef BT_PULL_LAUNCH
-    const bool vec = C == 1 && vec_neurons(d, z_given);
-    const dim3 vgrid(unsigned(ceil_div(n, 4 * kVecThreads)), unsigned(d.batch));
-    auto nvec = fast ? k_eng_neuron_vec<KIND, HARD, USE_REF, true> : k_eng_neuron_vec<KIND, HARD, USE_REF, false>;
   } else {
     const int grid = int(ceil_div(n, 32));
     const size_t smem = sizeof(uint32_t) * size_t(d.batch);
-      else if (vec) nvec<<<vgrid, kVecThreads, 0, s>>>(d, int(k), si, scatter_scratch(d, si.q_t), z_given);
     BT_CHECK_ARG(smem <= 48 * 1024, "batch too large for the gather engine");
     auto gather = n_rec(d) > 1 ? k_eng_gather<KIND, HARD, USE_REF, true> : k_eng_gather<KIND, HARD, USE_REF, false>;
     for (int64_t k = 0; k < d.n_steps; ++k)
@@ -1843,6 +1886,9 @@ int engine_run(const bt_engine_desc* d, const float* z_given, void* stream) {
   if (r) return run_typed<BT_NEURON_ALIF, false, true>(*d, z_given, s);
   return run_typed<BT_NEURON_ALIF, false, false>(*d, z_given, s);
 }
+}  // namespace
+
+extern "C" int bt_engine_run(const bt_engine_desc* d, void* stream) { return engine_run(d, nullptr, stream); }
 
 extern "C" int bt_engine_prime(const bt_engine_desc* d, void* stream) {
   if (int st = engine_check(d)) return st;
@@ -1886,9 +1932,6 @@ extern "C" int bt_input_project(int64_t rows, int64_t c_in, int64_t n, const flo
                                 const float* bias, float* out, int32_t* work, void* stream) {
   return input_project(rows, c_in, n, xin, w_t, bias, out, work, nullptr, 1, stream);
 }
-}  // namespace
-
-extern "C" int bt_engine_run(const bt_engine_desc* d, void* stream) { return engine_run(d, nullptr, stream); }
 
 extern "C" int bt_input_project_live(int64_t steps, int64_t batch, int64_t c_in, int64_t n, const float* xin,
                                      const float* w_t, const float* bias, const int32_t* sample_len, float* out,
