@@ -52,6 +52,31 @@ namespace bt {
 constexpr int kEngThreads = 256;
 constexpr int kMaxRec = 16;  // receptor channels per neuron
 
+// Programmatic dependent launch of the step kernels: a launch may be scheduled
+// as soon as every block of the one before it has started (step_begin signals
+// it), so its launch latency and the set-up of its blocks overlap the other's
+// tail; step_begin then waits for that grid to complete and its writes to be
+// visible before any global access.
+__device__ __forceinline__ void step_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_step(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // Receptor columns per neuron (0 in the descriptor means 1).
 __host__ __device__ __forceinline__ int n_rec(const bt_engine_desc& d) { return d.n_rec > 1 ? d.n_rec : 1; }
 
@@ -263,6 +288,7 @@ __device__ __forceinline__ void publish_spikes(const bt_engine_desc& d, const St
 // into the per-step input and trace arrays.
 template <int KIND, bool HARD, bool USE_REF, int S, bool FAST>
 __global__ void __launch_bounds__(kEngThreads) k_eng_neuron(bt_engine_desc d, int k, StepIdx si, ScatterScratch ws) {
+  step_begin();
   const int n = int(d.n), B = int(d.batch);
   const int words = (n + 31) >> 5;
   const int i = int(blockIdx.x) * kEngThreads + int(threadIdx.x);
@@ -413,6 +439,7 @@ constexpr int kVecThreads = 128;
 template <int KIND, bool HARD, bool USE_REF, bool FAST>
 __global__ void __launch_bounds__(kVecThreads) k_eng_neuron_vec(bt_engine_desc d, int k, StepIdx si, ScatterScratch ws,
                                                                 const float* __restrict__ z_given) {
+  step_begin();
   const int n = int(d.n), B = int(d.batch);
   const int words = (n + 31) >> 5;
   const int i0 = (int(blockIdx.x) * kVecThreads + int(threadIdx.x)) * 4;
@@ -521,6 +548,7 @@ __global__ void __launch_bounds__(kVecThreads) k_eng_neuron_vec(bt_engine_desc d
 // alias it waits for the store, which made this step latency bound.
 template <int KIND, bool HARD, bool USE_REF, int CT>
 __global__ void __launch_bounds__(kEngThreads) k_eng_neuron_rec(bt_engine_desc d, int64_t k, StepIdx si) {
+  step_begin();
   constexpr int M = CT > 0 ? CT : kMaxRec;
   const int64_t n = d.n, B = d.batch;
   const int C = CT > 0 ? CT : n_rec(d);
@@ -850,6 +878,7 @@ __device__ void scatter_dense(const bt_engine_desc& d, int64_t k, const ScatterS
 // has settled on 48 registers and spilled the reduction loop.
 template <int G, int MS>
 __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt_engine_desc d, int64_t k, StepIdx si) {
+  step_begin();
   extern __shared__ int32_t s_off[];  // [planes * kSub + 1]
   const int64_t n = d.n;
   const int R = d.n_bins, planes = d.bin_hi - d.bin_lo + 1;
@@ -966,6 +995,7 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
 template <int MS>
 __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_flat(bt_engine_desc d, int64_t k,
                                                                               StepIdx si) {
+  step_begin();
   extern __shared__ int32_t s_off[];  // [planes * kSub + 1]
   const int R = d.n_bins, planes = d.bin_hi - d.bin_lo + 1;
   const ScatterScratch ws0 = scatter_scratch(d, 0);
@@ -1806,10 +1836,10 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
     auto nvec = fast ? k_eng_neuron_vec<KIND, HARD, USE_REF, true> : k_eng_neuron_vec<KIND, HARD, USE_REF, false>;
     for (int64_t k = 0; k < d.n_steps; ++k) {
       const StepIdx si = step_idx(d.t0 + k, d.n_bins, d.hist_len);
-      if (C > 1) rec<<<rgrid, kEngThreads, 0, s>>>(d, k, si);
-      else if (vec) nvec<<<vgrid, kVecThreads, 0, s>>>(d, int(k), si, scatter_scratch(d, si.q_t), z_given);
-      else neuron<<<grid, kEngThreads, 0, s>>>(d, int(k), si, scatter_scratch(d, si.q_t));
-      scatter<<<sgrid, kEngThreads, ssmem, s>>>(d, k, si);
+      if (C > 1) launch_step(rec, rgrid, kEngThreads, 0, s, d, k, si);
+      else if (vec) launch_step(nvec, vgrid, kVecThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
+      else launch_step(neuron, grid, kEngThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t));
+      launch_step(scatter, dim3(sgrid), kEngThreads, ssmem, s, d, k, si);
     }
     BT_CHECK_LAUNCH("k_eng_neuron/k_eng_scatter");
     if (d.n_steps > 0) {
