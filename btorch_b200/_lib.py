@@ -90,6 +90,9 @@ _PROTOS = {
     "bt_input_project_live": (C.c_int, [_i64, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bt_bits_to_float": (C.c_int, [_i64, _i64, _vp, _vp, _vp]),
     "bt_float_to_bits": (C.c_int, [_i64, _i64, _vp, _vp, _vp]),
+    "bt_history_load": (C.c_int, [_i64, _i32, _i64, _vp, _vp, _i64, _i32, _vp, _vp]),
+    "bt_history_store": (C.c_int, [_i64, _i32, _i64, _vp, _i64, _i32, _vp, _i64, _vp, _vp]),
+    "bt_pack_edges": (C.c_int, [_i64, _i64, _vp, _vp, _vp, _vp, _vp]),
     "bt_raster_count": (C.c_int, [_i64, _i64, _vp, _vp, _vp]),
     "bt_raster_coords": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bt_float_to_masks": (C.c_int, [_i64, _i64, _vp, _vp, _vp]),

@@ -115,6 +115,20 @@ def pack_csr_weights(layout: SparseLayout, w_canonical: torch.Tensor) -> torch.T
     return out
 
 
+def pack_edges(layout: SparseLayout, w_canonical: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """The (post, weight) records of the CSR view (bt_engine_desc.csr_edges),
+    padded like csr_dst."""
+    perm = getattr(layout, "csr_perm32", None)
+    if perm is None:
+        perm = layout.csr_perm32 = layout.csr_perm.to(torch.int32)
+    if out is None:
+        out = torch.empty(2 * layout.csr_dst.numel(), device=w_canonical.device, dtype=torch.int32)
+    L.check(L.lib().bt_pack_edges(layout.nnz, layout.csr_dst.numel(), layout.csr_dst.data_ptr(), perm.data_ptr(),
+                                  w_canonical.data_ptr(), out.data_ptr(), L.stream_of(w_canonical.device)),
+            "bt_pack_edges")
+    return out
+
+
 # ---------------------------------------------------------- sparse product --
 
 

@@ -25,7 +25,7 @@ from .. import _lib as L
 from . import autotune as _autotune
 from . import environ
 from . import _ops
-from ._ops import build_slices, neuron_desc, pack_csr_weights, pack_slice_weights, scalar_values
+from ._ops import build_slices, neuron_desc, pack_edges, pack_slice_weights, scalar_values
 from .functional import named_hidden_states
 from .history import SpikeHistory
 from .linear import BaseSparseConn
@@ -482,17 +482,19 @@ def run(plan: EnginePlan, rnn, x: torch.Tensor, sample_len: torch.Tensor | None 
         desc.psc_fast_div, desc.psc_rcp = int(ok), r
     desc.mode = mode
     lay = conn.engine_layout(R, plan.uniform_delay, dev)
-    w = static("w", conn._edge_weight().detach().float().contiguous())
+    w = conn._edge_weight().detach().float().contiguous()
+    if mode != L.BT_MODE_SCATTER:  # (scatter reads the edge records packed from it)
+        w = static("w", w)
     keep.append(w)
     desc.n, desc.batch, desc.n_bins, desc.n_rec = n, B, R, n_rec
     desc.hist_len = H
-    desc.csc_ptr, desc.csc_src, desc.csc_w = lay.csc_ptr.data_ptr(), lay.csc_src.data_ptr(), w.data_ptr()
+    desc.csc_ptr, desc.csc_src = lay.csc_ptr.data_ptr(), lay.csc_src.data_ptr()
+    desc.csc_w = w.data_ptr() if mode != L.BT_MODE_SCATTER else None
     if mode == L.BT_MODE_SCATTER:
         lay_s = conn.scatter_layout(R, plan.uniform_delay, dev)
-        w_csr = pack_csr_weights(lay_s, w)
         # one (post, weight) record per edge, interleaved
-        edges = static("csr_edges", torch.stack([lay_s.csr_dst, w_csr.view(torch.int32)], 1).reshape(-1))
-        keep += [w_csr, edges]
+        edges = pack_edges(lay_s, w, alloc("csr_edges", (2 * lay_s.csr_dst.numel(),), torch.int32))
+        keep.append(edges)
         desc.csr_ptr, desc.csr_edges = lay_s.csr_ptr.data_ptr(), edges.data_ptr()
         desc.bin_lo, desc.bin_hi = lay_s.bin_lo, lay_s.bin_hi
         desc.scatter_lanes = choice.scatter_lanes or (1 if lay_s.mean_row < 48 else 32)
@@ -516,8 +518,7 @@ def run(plan: EnginePlan, rnn, x: torch.Tensor, sample_len: torch.Tensor | None 
     tile_ws = None
     if mode == L.BT_MODE_TILE:
         lay_s = conn.scatter_layout(R, plan.uniform_delay, dev)
-        w_csr = pack_csr_weights(lay_s, w)
-        edges = static("csr_edges", torch.stack([lay_s.csr_dst, w_csr.view(torch.int32)], 1).reshape(-1))
+        edges = pack_edges(lay_s, w, alloc("csr_edges", (2 * lay_s.csr_dst.numel(),), torch.int32))
         shape = tile_shape(n, B, dev, choice.tile_posts)
         if shape is None:
             raise NotImplementedError("tile mode: the tile accumulators do not fit in shared memory")
@@ -525,7 +526,7 @@ def run(plan: EnginePlan, rnn, x: torch.Tensor, sample_len: torch.Tensor | None 
         toff = tile_offsets(lay_s, edges, tp, P, dev)
         ring = alloc("ring", (B, nc), torch.float32, zero=True)  # W z handed to the final launch
         tile_ws = alloc("tile_work", (L.lib().bt_tile_work_words(B, tp, P),), torch.int32, zero=True)
-        keep += [w_csr, edges, ring, tile_ws, toff]
+        keep += [edges, ring, tile_ws, toff]
         desc.csr_ptr, desc.csr_edges, desc.ring = lay_s.csr_ptr.data_ptr(), edges.data_ptr(), ring.data_ptr()
         desc.bin_lo = desc.bin_hi = 0
         desc.tile_posts, desc.n_tiles = tp, P
@@ -583,17 +584,13 @@ def run(plan: EnginePlan, rnn, x: torch.Tensor, sample_len: torch.Tensor | None 
     hist_depth = plan.history.max_delay if plan.history is not None else 0
     want_hist_trace = "history" in plan.paths.values()
     if hist_depth:
-        block = plan.history.recent_block(hist_depth).float().contiguous()  # [Dh, B, n], d steps ago
         if mode == L.BT_MODE_PULL:
+            block = plan.history.recent_block(hist_depth).float().contiguous()  # [Dh, B, n], d steps ago
             for d in range(hist_depth):
                 L.check(L.lib().bt_float_to_masks(B, n, block[d].data_ptr(), masks[(t0 - 1 - d) % H].data_ptr(), s),
                         "bt_float_to_masks")
         else:
-            bits = torch.empty((hist_depth, B, words), device=dev, dtype=torch.int32)
-            L.check(L.lib().bt_float_to_bits(hist_depth * B, n, block.data_ptr(), bits.data_ptr(), s),
-                    "bt_float_to_bits")
-            for d in range(hist_depth):
-                hist[(t0 - 1 - d) % H] = bits[d]
+            plan.history.to_ring(hist, B, t0)
     desc.t0 = t0
     if mode == L.BT_MODE_SCATTER:
         # spike sets of the history steps whose arrivals are still pending
@@ -814,17 +811,15 @@ def run(plan: EnginePlan, rnn, x: torch.Tensor, sample_len: torch.Tensor | None 
     # write the spike history back into the module (last Dh spikes)
     t_end = t0 + T
     if hist_depth:
-        block = torch.empty((hist_depth, B, n), device=dev, dtype=torch.float32)
+        init_block = plan.history.recent_block(hist_depth).clone() if want_hist_trace else None
         if mode == L.BT_MODE_PULL:
+            block = torch.empty((hist_depth, B, n), device=dev, dtype=torch.float32)
             for d in range(hist_depth):
                 L.check(L.lib().bt_masks_to_float(B, n, masks[(t_end - 1 - d) % H].data_ptr(), block[d].data_ptr(), s),
                         "bt_masks_to_float")
+            plan.history.store_recent_block(block, T)
         else:
-            sel = torch.stack([hist[(t_end - 1 - d) % H] for d in range(hist_depth)]).contiguous()
-            L.check(L.lib().bt_bits_to_float(hist_depth * B, n, sel.data_ptr(), block.data_ptr(), s),
-                    "bt_bits_to_float")
-        init_block = plan.history.recent_block(hist_depth).clone() if want_hist_trace else None
-        plan.history.store_recent_block(block, T)
+            plan.history.from_ring(hist, B, t_end, T)
     if plan.hetero:
         lead = psc_mod.psc.shape[:-1]
         if n_rec == 1:

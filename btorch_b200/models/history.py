@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import torch
 
+from .. import _lib as L
 from .base import MemoryModule, normalize_n_neuron
 
 
@@ -105,3 +106,46 @@ class SpikeHistory(MemoryModule):
             h[order] = new
         else:
             self.history = new.movedim(0, nb).contiguous() if nb > 0 else new.clone()
+
+    def _kernel_state(self, batch: int) -> bool:
+        """The history is [batch][max_delay][n] contiguous fp32 on the device."""
+        h = self.history
+        return (h.is_cuda and h.dtype == torch.float32 and h.is_contiguous()
+                and h.numel() == batch * self.max_delay * self.size
+                and (not self.use_circular_buffer or self._cursor.device == h.device))
+
+    def to_ring(self, ring: torch.Tensor, batch: int, t0: int) -> None:
+        """The spikes d = 0 .. max_delay - 1 steps ago as bitmaps in slots
+        (t0 - 1 - d) mod H of the engine's history ring [H][batch][words]."""
+        H, words = ring.shape[0], ring.shape[-1]
+        s = L.stream_of(ring.device)
+        if self._kernel_state(batch):
+            cursor = self._cursor.data_ptr() if self.use_circular_buffer else None
+            L.check(L.lib().bt_history_load(batch, self.max_delay, self.size, self.history.data_ptr(), cursor, t0, H,
+                                            ring.data_ptr(), s), "bt_history_load")
+            return
+        block = self.recent_block(self.max_delay).float().contiguous()
+        bits = torch.empty((self.max_delay, batch, words), device=ring.device, dtype=torch.int32)
+        L.check(L.lib().bt_float_to_bits(self.max_delay * batch, self.size, block.data_ptr(), bits.data_ptr(), s),
+                "bt_float_to_bits")
+        for d in range(self.max_delay):
+            ring[(t0 - 1 - d) % H] = bits[d]
+
+    def from_ring(self, ring: torch.Tensor, batch: int, t_end: int, advance: int) -> None:
+        """The state after `advance` steps from the ring's bitmaps of steps
+        t_end - 1 - d (as store_recent_block)."""
+        H = ring.shape[0]
+        s = L.stream_of(ring.device)
+        if self._kernel_state(batch):
+            if self.use_circular_buffer:
+                cursor = self._cursor.data_ptr()
+            else:
+                cursor, self.history = None, torch.empty_like(self.history)
+            L.check(L.lib().bt_history_store(batch, self.max_delay, self.size, ring.data_ptr(), t_end, H, cursor,
+                                             advance, self.history.data_ptr(), s), "bt_history_store")
+            return
+        block = torch.empty((self.max_delay, batch, self.size), device=ring.device, dtype=torch.float32)
+        sel = torch.stack([ring[(t_end - 1 - d) % H] for d in range(self.max_delay)]).contiguous()
+        L.check(L.lib().bt_bits_to_float(self.max_delay * batch, self.size, sel.data_ptr(), block.data_ptr(), s),
+                "bt_bits_to_float")
+        self.store_recent_block(block, advance)

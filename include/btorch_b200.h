@@ -531,6 +531,23 @@ BT_API int bt_raster_coords(int64_t rows, int64_t batch, int64_t n, const uint32
                             const int64_t* offsets, int32_t* idx_time, int32_t* idx_batch,
                             int32_t* idx_neuron, void* stream);
 
+/* A module's spike history (SpikeHistory, btorch/models/history.py:28-358) to
+ * and from the engine's bitmap ring.  hist: [batch][D][n] fp32; cursor: device
+ * int64, the spikes d steps ago in slot (cursor - 1 - d) mod D, or NULL: in
+ * slot d.  bt_history_load writes ring slots (t0 - 1 - d) mod H, d < D.
+ * bt_history_store sets hist to the spikes of steps t_end - 1 - d and advances
+ * the cursor by `advance`. */
+BT_API int bt_history_load(int64_t batch, int32_t D, int64_t n, const float* hist, const int64_t* cursor,
+                           int64_t t0, int32_t H, uint32_t* ring, void* stream);
+BT_API int bt_history_store(int64_t batch, int32_t D, int64_t n, const uint32_t* ring, int64_t t_end, int32_t H,
+                            int64_t* cursor, int64_t advance, float* hist, void* stream);
+
+/* bt_engine_desc.csr_edges from the CSR view: record e = (csr_dst[e], the bits
+ * of w[csr_perm[e]]), weight 0 for nnz <= e < padded (padded a multiple of 4,
+ * the length of csr_dst; csr_dst and edges 16-byte aligned). */
+BT_API int bt_pack_edges(int64_t nnz, int64_t padded, const uint32_t* csr_dst, const int32_t* csr_perm,
+                         const float* w, uint32_t* edges, void* stream);
+
 BT_API int bt_float_to_bits(int64_t rows, int64_t n, const float* in,
                      uint32_t* bits, void* stream);
 
