@@ -65,6 +65,18 @@ class BtEngineDesc(C.Structure):
     ]
 
 
+class BtBpttDesc(C.Structure):
+    _fields_ = [
+        ("batch", _i64), ("n", _i64), ("n_steps", _i64),
+        ("neuron", BtNeuronDesc), ("psc_coef", BtParam), ("psc_tau", BtParam), ("detach_reset", _i32), ("pad_", _i32),
+        ("csr_ptr", _vp), ("csr_dst", _vp), ("csr_w", _vp),
+        ("x", _vp), ("z", _vp), ("v", _vp), ("psc", _vp), ("ref", _vp), ("gk", _vp),
+        ("g_z", _vp), ("g_v", _vp), ("g_psc", _vp), ("g_gk", _vp),
+        ("cur_psc", _vp), ("cur_v", _vp), ("cur_gk", _vp),
+        ("G_psc", _vp), ("G_I", _vp), ("gz", _vp), ("gT", _vp),
+    ]
+
+
 _PROTOS = {
     "bt_last_error": (C.c_char_p, []),
     "bt_abi_version": (C.c_int, []),
@@ -85,6 +97,8 @@ _PROTOS = {
     "bt_neuron_step_backward": (C.c_int, [C.POINTER(BtNeuronDesc), _i64, _i64] + [_vp] * 13 + [_i32, _vp]),
     "bt_psc_step": (C.c_int, [_i64, _i64, BtParam, BtParam, _vp, _vp, _vp, _vp]),
     "bt_engine_run": (C.c_int, [C.POINTER(BtEngineDesc), _vp]),
+    "bt_engine_run_given": (C.c_int, [C.POINTER(BtEngineDesc), _vp, _vp]),
+    "bt_bptt_backward": (C.c_int, [C.POINTER(BtBpttDesc), _vp]),
     "bt_engine_prime": (C.c_int, [C.POINTER(BtEngineDesc), _vp]),
     "bt_input_project": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bt_input_project_live": (C.c_int, [_i64, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),

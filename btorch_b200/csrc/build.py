@@ -18,8 +18,8 @@ PKG = CSRC.parent
 ROOT = PKG.parent
 LIB_DIR = PKG / "_lib"
 LIB = LIB_DIR / "libbtorch_b200.so"
-SOURCES = ["layout.cpp", "spmv.cu", "spmm.cu", "gradw.cu", "neuron.cu", "engine.cu", "tile.cu", "cluster.cu", "raster.cu", "history.cu"]
-HEADERS = ["common.cuh", "neuron.cuh"]
+SOURCES = ["layout.cpp", "spmv.cu", "spmm.cu", "gradw.cu", "neuron.cu", "engine.cu", "tile.cu", "cluster.cu", "raster.cu", "history.cu", "bptt.cu"]
+HEADERS = ["common.cuh", "neuron.cuh", "neuron_backward.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

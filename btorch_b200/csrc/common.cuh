@@ -157,4 +157,29 @@ inline void launch_setup_add(const void* kern, int dev, size_t smem, int blocks)
   launch_setups().push_back(LaunchSetup{kern, dev, smem, blocks});
 }
 
+// Programmatic dependent launch of the step kernels: a launch may be scheduled
+// as soon as every block of the one before it has started (step_begin signals
+// it), so its launch latency and the set-up of its blocks overlap the other's
+// tail; step_begin then waits for that grid to complete and its writes to be
+// visible before any global access.
+__device__ __forceinline__ void step_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_step(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 }  // namespace bt

@@ -52,31 +52,6 @@ namespace bt {
 constexpr int kEngThreads = 256;
 constexpr int kMaxRec = 16;  // receptor channels per neuron
 
-// Programmatic dependent launch of the step kernels: a launch may be scheduled
-// as soon as every block of the one before it has started (step_begin signals
-// it), so its launch latency and the set-up of its blocks overlap the other's
-// tail; step_begin then waits for that grid to complete and its writes to be
-// visible before any global access.
-__device__ __forceinline__ void step_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename... P, typename... A>
-cudaError_t launch_step(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(unsigned(threads));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
-}
-
 // Receptor columns per neuron (0 in the descriptor means 1).
 __host__ __device__ __forceinline__ int n_rec(const bt_engine_desc& d) { return d.n_rec > 1 ? d.n_rec : 1; }
 
@@ -287,7 +262,8 @@ __device__ __forceinline__ void publish_spikes(const bt_engine_desc& d, const St
 // are 32-bit (batch * n < 2^31 in scatter mode, checked on the host) except
 // into the per-step input and trace arrays.
 template <int KIND, bool HARD, bool USE_REF, int S, bool FAST>
-__global__ void __launch_bounds__(kEngThreads) k_eng_neuron(bt_engine_desc d, int k, StepIdx si, ScatterScratch ws) {
+__global__ void __launch_bounds__(kEngThreads) k_eng_neuron(bt_engine_desc d, int k, StepIdx si, ScatterScratch ws,
+                                                          const float* __restrict__ z_given) {
   step_begin();
   const int n = int(d.n), B = int(d.batch);
   const int words = (n + 31) >> 5;
@@ -378,6 +354,8 @@ __global__ void __launch_bounds__(kEngThreads) k_eng_neuron(bt_engine_desc d, in
       hist_p[u * words] = word;
       if (raster_p) raster_p[u * words] = word;
     }
+    // z_given: publish these spikes instead of the step's own
+    if (z_given && valid) s = z_given[(int64_t(k) * B + b0 + u) * n + i];
     if (s != 0.0f) spiked |= 1u << u;
   }
   publish_spikes_ws(ws, i, b0, spiked);
@@ -1838,7 +1816,7 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
       const StepIdx si = step_idx(d.t0 + k, d.n_bins, d.hist_len);
       if (C > 1) launch_step(rec, rgrid, kEngThreads, 0, s, d, k, si);
       else if (vec) launch_step(nvec, vgrid, kVecThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
-      else launch_step(neuron, grid, kEngThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t));
+      else launch_step(neuron, grid, kEngThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
       launch_step(scatter, dim3(sgrid), kEngThreads, ssmem, s, d, k, si);
     }
     BT_CHECK_LAUNCH("k_eng_neuron/k_eng_scatter");
@@ -1919,6 +1897,12 @@ int engine_run(const bt_engine_desc* d, const float* z_given, void* stream) {
 }  // namespace
 
 extern "C" int bt_engine_run(const bt_engine_desc* d, void* stream) { return engine_run(d, nullptr, stream); }
+
+extern "C" int bt_engine_run_given(const bt_engine_desc* d, const float* spikes, void* stream) {
+  if (spikes && d && (d->mode != BT_MODE_SCATTER || d->n_rec > 1))
+    return bt_set_error(BT_ERR_UNSUPPORTED, "given spikes need the scatter mode without receptor channels");
+  return engine_run(d, spikes, stream);
+}
 
 extern "C" int bt_engine_prime(const bt_engine_desc* d, void* stream) {
   if (int st = engine_check(d)) return st;

@@ -1,6 +1,6 @@
 // Single-step neuron and synapse kernels (the per-module path used when a
 // model is stepped module by module, and for autograd).
-#include "neuron.cuh"
+#include "neuron_backward.cuh"
 
 namespace bt {
 
@@ -25,9 +25,6 @@ __global__ void k_neuron_step(bt_neuron_desc d, int64_t batch, int64_t n, const 
   if (vch_save) vch_save[idx] = o.v_charged;
 }
 
-// Reverse-mode derivative of one neuron step, following the autograd graph
-// the reference builds from its eager ops.  The fire step's surrogate is the
-// sigmoid one: damping * 4 * s(k a u) * (1 - s(k a u)).
 __global__ void k_neuron_step_backward(bt_neuron_desc d, int64_t batch, int64_t n, const float* x,
                                        const float* g_spike, const float* g_v_new, const float* g_gk_new,
                                        const float* u_save, const float* spike, const float* mask_save,
@@ -36,54 +33,15 @@ __global__ void k_neuron_step_backward(bt_neuron_desc d, int64_t batch, int64_t 
   const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= batch * n) return;
   const int64_t i = idx % n;
-  const float vth = ld(d.v_threshold, i), vr = ld(d.v_reset, i), cm = ld(d.c_m, i);
-  const float dt = d.dt;
-  const float s = spike[idx], u = u_save[idx], mask = mask_save[idx], v1 = v_charged[idx];
-  const float gv2 = g_v_new ? g_v_new[idx] : 0.0f;
   const bool alif = d.kind == BT_NEURON_ALIF;
-  const float ggk2 = (alif && g_gk_new) ? g_gk_new[idx] : 0.0f;
-  float gs = g_spike ? g_spike[idx] : 0.0f;
-  const float den = vth - vr;
-  // reset:  hard v2 = v1 - (v1 - vr) * s ;  soft v2 = v1 - (vth - vr) * s
-  float gv1, gs_reset;
-  if (d.hard_reset) {
-    gv1 = gv2 - gv2 * s;
-    gs_reset = -gv2 * (v1 - vr);
-  } else {
-    gv1 = gv2;
-    gs_reset = -gv2 * den;
-  }
-  if (alif) gs_reset += ggk2 * ld(d.dg_k, i);  // gk2 = gk1 + dg_k * s
-  if (!detach_reset) gs += gs_reset;
-  // fire:  s = H(u) * mask with the surrogate derivative at u;  u = (v1 - vth) / den
-  const float sig = sigmoidf_dev(d.sg_alpha * u);
-  const float gu = (gs * mask) * (d.sg_damping * 4.0f * sig * (1.0f - sig));
-  gv1 += gu / den;
-  const float v = v_prev[idx];
-  if (!alif) {
-    // charge: v1 = v + dt * ((-(v - vr)) / tau + I / cm)
-    const float gD = dt * gv1;
-    g_x[idx] = gD / cm;
-    if (g_v_prev) g_v_prev[idx] = gv1 - gD / ld(d.tau, i);
-    return;
-  }
-  // charge: v1 = v + C(lin) * D,  D = (ngl (v - El) + (-gk)(v - Ek) + I) / cm,  lin = (ngl - gk) / cm
-  const float gk = gk_prev[idx];
-  const float ngl = -ld(d.g_leak, i);
-  const float Ek = ld(d.E_k, i);
-  const float lin = (ngl - gk) / cm;
-  const float em1 = expm1f(dt * lin);
-  const float C = em1 / lin;
-  const float D = (ngl * (v - ld(d.E_leak, i)) + (-gk) * (v - Ek) + x[idx]) / cm;
-  const float gC = gv1 * D, gD = gv1 * C;
-  g_x[idx] = gD / cm;
-  if (g_v_prev) g_v_prev[idx] = gv1 + gD * lin;
-  // dC/dlin = (dt e^{dt lin} lin - expm1(dt lin)) / lin^2 ; dlin/dgk = -1/cm ; dD/dgk = -(v - Ek)/cm
-  const float dCdl = (dt * (em1 + 1.0f) * lin - em1) / (lin * lin);
-  const float g_gk_charge = -(gC * dCdl) / cm - gD * (v - Ek) / cm;
-  // adaptation: gk1 = gk + coef_gk * ((-gk) / tau_adapt)
-  const float dgk1 = 1.0f - ld(d.coef_gk, i) / ld(d.tau_adapt, i);
-  if (g_gk_prev) g_gk_prev[idx] = ggk2 * dgk1 + g_gk_charge;
+  const NeuronParams p = alif ? load_params<BT_NEURON_ALIF, false>(d, i) : load_params<BT_NEURON_LIF, false>(d, i);
+  const NeuronGrad o = neuron_backward(
+      p, d.sg_damping, alif, d.hard_reset != 0, detach_reset != 0, g_spike ? g_spike[idx] : 0.0f,
+      g_v_new ? g_v_new[idx] : 0.0f, (alif && g_gk_new) ? g_gk_new[idx] : 0.0f, x[idx], v_prev[idx],
+      alif ? gk_prev[idx] : 0.0f, spike[idx], u_save[idx], mask_save[idx], v_charged[idx]);
+  g_x[idx] = o.x;
+  if (g_v_prev) g_v_prev[idx] = o.v;
+  if (alif && g_gk_prev) g_gk_prev[idx] = o.gk;
 }
 
 __global__ void k_psc_step(int64_t batch, int64_t n, bt_param coef, bt_param tau, const float* psc,

@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32) k_rows_gather(int64_t batch
                                                                   const uint32_t* __restrict__ col,
                                                                   const float* __restrict__ wts,
                                                                   const float* __restrict__ gT, float* __restrict__ out) {
+  step_begin();
   constexpr int S = 32 / G, R = kGatherWarps / P;  // lane groups of a warp, rows of a CTA
   __shared__ float s_out[kGatherWarps][G * V + 1];
   const int warp = int(threadIdx.x >> 5), lane = int(lane_id());
@@ -129,8 +130,8 @@ static void launch_gather_g(int64_t batch, int64_t pitch, int64_t n_rows, const 
                             const float* wts, const float* gT, float* out, cudaStream_t s) {
   const int64_t ny = ceil_div(pitch, G * V);
   auto go = [&](auto kern, int P) {
-    kern<<<dim3(unsigned(ceil_div(n_rows, kGatherWarps / P)), unsigned(ny)), kGatherWarps * 32, 0, s>>>(
-        batch, pitch, n_rows, ptr, col, wts, gT, out);
+    launch_step(kern, dim3(unsigned(ceil_div(n_rows, kGatherWarps / P)), unsigned(ny)), kGatherWarps * 32, 0, s, batch,
+                pitch, n_rows, ptr, col, wts, gT, out);
   };
   const int64_t warps = n_rows * ny, want = 148 * 40;
   if (warps >= want) go(k_rows_gather<V, G, 1>, 1);

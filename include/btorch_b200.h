@@ -485,6 +485,43 @@ BT_API int bt_engine_run(const bt_engine_desc* d, void* stream);
  * at the start of a multi-step call. */
 BT_API int bt_engine_prime(const bt_engine_desc* d, void* stream);
 
+/* bt_engine_run (scatter mode, no receptor channels) with the recurrent input
+ * driven by given spikes [n_steps][batch][n] (fp32, nonzero = a spike) instead of
+ * the steps' own, which still reset their neurons: the recomputation of a
+ * checkpointed run, whatever the order its sums were formed in.  NULL: plain
+ * bt_engine_run. */
+BT_API int bt_engine_run_given(const bt_engine_desc* d, const float* spikes, void* stream);
+
+/* Backward of n_steps steps of LIF / ALIF + ExponentialPSC over a square
+ * connection (n posts, n sources), surrogate gradients as
+ * bt_neuron_step_backward.  All arrays fp32; G_* and g_* of step t at
+ * [t][batch][n]. */
+typedef struct bt_bptt_desc {
+  int64_t batch, n, n_steps;
+  bt_neuron_desc neuron;          /* spiking = 1 */
+  bt_param psc_coef, psc_tau;
+  int32_t detach_reset;
+  int32_t pad_;
+  /* CSR by source, csr_dst = post, csr_w in CSR order */
+  const int32_t* csr_ptr; const uint32_t* csr_dst; const float* csr_w;
+  /* the forward: drive x [n_steps] (the input current without the PSC), spikes
+     z [n_steps]; state [n_steps + 1] before step 0 and after every step (ref
+     NULL without refractory, gk NULL unless ALIF) */
+  const float *x, *z;
+  const float *v, *psc, *ref, *gk;
+  /* gradients of the returned spikes and state stacks, [n_steps] each, may be NULL */
+  const float *g_z, *g_v, *g_psc, *g_gk;
+  /* [batch][n], in: gradient of the state after the last step, out: of the
+     state before the first (cur_gk: ALIF) */
+  float *cur_psc, *cur_v, *cur_gk;
+  /* out, [n_steps] each: gradient of the PSC after every step, of the input
+     current of every step (G_I may alias x) */
+  float *G_psc, *G_I;
+  /* scratch: [batch][n], and [n][4 * ceil(batch / 4)], 16-byte aligned */
+  float *gz, *gT;
+} bt_bptt_desc;
+BT_API int bt_bptt_backward(const bt_bptt_desc* d, void* stream);
+
 /* Input projection for DenseConn as neuron_inp_module (nn.Linear,
  * btorch/models/linear.py:163-228): out[r, i] = bias[i] + sum over nonzero
  * xin[r, c] (ascending c) of xin[r, c] * w_t[c, i].  rows = steps*batch;
