@@ -84,6 +84,8 @@ _PROTOS = {
     "bt_layout_slices": (C.c_int, [_i64, _vp, _vp, C.c_uint32, _vp, _vp, _vp, _i64, _vp]),
     "bt_spmv_gather": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bt_spmv_scatter": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "bt_spmv_push_work_words": (C.c_int64, [_i64, _i64, _i64]),
+    "bt_spmv_push": (C.c_int, [_i64, _i64, _i64, _i64] + [_vp] * 11),
     "bt_spmv_gather_noalloc": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bt_spmv_grad_input": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bt_spmv_grad_input_t": (C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),

@@ -4,6 +4,9 @@
 // contiguous run of samples instead of one scattered word per sample.  Used
 // by the backward of SparseConn (rows = sources, columns = posts; the
 // reference's torch index-op backward, btorch/models/_sparse_triton.py:389-415).
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace bt {
@@ -62,13 +65,11 @@ constexpr int kGatherWarps = 8;
 // shared memory, as runs of out[b].  Measured and slower: streaming gT
 // through shared memory in column tiles (195 us), and narrow sample blocks
 // with several rows per warp for reuse in L1 (150 us).
-template <int V, int G, int P>
-__global__ void __launch_bounds__(kGatherWarps * 32) k_rows_gather(int64_t batch, int64_t pitch, int64_t n_rows,
-                                                                  const int32_t* __restrict__ ptr,
-                                                                  const uint32_t* __restrict__ col,
-                                                                  const float* __restrict__ wts,
-                                                                  const float* __restrict__ gT, float* __restrict__ out) {
-  step_begin();
+// SKIP0: entries of gT that are zero add nothing, whatever the weight.
+template <int V, int G, int P, bool SKIP0>
+__device__ __forceinline__ void rows_gather(int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* __restrict__ ptr,
+                                            const uint32_t* __restrict__ col, const float* __restrict__ wts,
+                                            const float* __restrict__ gT, float* __restrict__ out) {
   constexpr int S = 32 / G, R = kGatherWarps / P;  // lane groups of a warp, rows of a CTA
   __shared__ float s_out[kGatherWarps][G * V + 1];
   const int warp = int(threadIdx.x >> 5), lane = int(lane_id());
@@ -98,7 +99,8 @@ __global__ void __launch_bounds__(kGatherWarps * 32) k_rows_gather(int64_t batch
         if (in && k < cnt) {
           const FVec<V> g = ld_vec<V>(gT + int64_t(cq) * pitch + bl);
 #pragma unroll
-          for (int v = 0; v < V; ++v) acc[v] = fmaf(wq, g.v[v], acc[v]);
+          for (int v = 0; v < V; ++v)
+            if (!SKIP0 || g.v[v] != 0.0f) acc[v] = fmaf(wq, g.v[v], acc[v]);
         }
       }
     }
@@ -122,46 +124,186 @@ __global__ void __launch_bounds__(kGatherWarps * 32) k_rows_gather(int64_t batch
   }
 }
 
+template <int V, int G, int P>
+__global__ void __launch_bounds__(kGatherWarps * 32) k_rows_gather(int64_t batch, int64_t pitch, int64_t n_rows,
+                                                                  const int32_t* __restrict__ ptr,
+                                                                  const uint32_t* __restrict__ col,
+                                                                  const float* __restrict__ wts,
+                                                                  const float* __restrict__ gT, float* __restrict__ out) {
+  step_begin();
+  rows_gather<V, G, P, false>(batch, pitch, n_rows, ptr, col, wts, gT, out);
+}
+
 // Warps per row: enough for about 40 warps per SM over the rows and sample
 // blocks (8192 rows: one; 4200 rows: 2, 1000 rows: 8; measured faster
 // than one, 8192 rows slower).
-template <int V, int G>
-static void launch_gather_g(int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* ptr, const uint32_t* col,
-                            const float* wts, const float* gT, float* out, cudaStream_t s) {
+template <int V, int G, typename F>
+static void pick_parts(int64_t pitch, int64_t n_rows, F&& go) {
   const int64_t ny = ceil_div(pitch, G * V);
-  auto go = [&](auto kern, int P) {
-    launch_step(kern, dim3(unsigned(ceil_div(n_rows, kGatherWarps / P)), unsigned(ny)), kGatherWarps * 32, 0, s, batch,
-                pitch, n_rows, ptr, col, wts, gT, out);
-  };
   const int64_t warps = n_rows * ny, want = 148 * 40;
-  if (warps >= want) go(k_rows_gather<V, G, 1>, 1);
-  else if (2 * warps >= want) go(k_rows_gather<V, G, 2>, 2);
-  else if (4 * warps >= want) go(k_rows_gather<V, G, 4>, 4);
-  else go(k_rows_gather<V, G, 8>, 8);
+  using std::integral_constant;
+  const integral_constant<int, V> v;
+  const integral_constant<int, G> g;
+  if (warps >= want) go(v, g, integral_constant<int, 1>(), ny);
+  else if (2 * warps >= want) go(v, g, integral_constant<int, 2>(), ny);
+  else if (4 * warps >= want) go(v, g, integral_constant<int, 4>(), ny);
+  else go(v, g, integral_constant<int, 8>(), ny);
 }
 
-template <int V>
-static void launch_gather(int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* ptr, const uint32_t* col,
-                          const float* wts, const float* gT, float* out, cudaStream_t s) {
+// go(V, G, P, sample blocks) for this shape
+template <int V, typename F>
+static void pick_lanes(int64_t pitch, int64_t n_rows, F&& go) {
   const int64_t nv = pitch / V;  // vectors of a row
-  if (nv <= 1) launch_gather_g<V, 1>(batch, pitch, n_rows, ptr, col, wts, gT, out, s);
-  else if (nv <= 2) launch_gather_g<V, 2>(batch, pitch, n_rows, ptr, col, wts, gT, out, s);
-  else if (nv <= 4) launch_gather_g<V, 4>(batch, pitch, n_rows, ptr, col, wts, gT, out, s);
-  else if (nv <= 8) launch_gather_g<V, 8>(batch, pitch, n_rows, ptr, col, wts, gT, out, s);
-  else if (nv <= 16) launch_gather_g<V, 16>(batch, pitch, n_rows, ptr, col, wts, gT, out, s);
-  else launch_gather_g<V, 32>(batch, pitch, n_rows, ptr, col, wts, gT, out, s);
+  if (nv <= 1) pick_parts<V, 1>(pitch, n_rows, go);
+  else if (nv <= 2) pick_parts<V, 2>(pitch, n_rows, go);
+  else if (nv <= 4) pick_parts<V, 4>(pitch, n_rows, go);
+  else if (nv <= 8) pick_parts<V, 8>(pitch, n_rows, go);
+  else if (nv <= 16) pick_parts<V, 16>(pitch, n_rows, go);
+  else pick_parts<V, 32>(pitch, n_rows, go);
 }
 
 // out [batch][n_rows] from gT [n_cols][pitch] (pitch >= batch, zeros past it).
 int rows_product(int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* ptr, const uint32_t* col,
                  const float* wts, const float* gT, float* out, cudaStream_t s) {
-  // the scratch of one that is not a multiple of 4, or not aligned, takes words
-  if (pitch % 4 == 0 && (reinterpret_cast<uintptr_t>(gT) & 15) == 0)
-    launch_gather<4>(batch, pitch, n_rows, ptr, col, wts, gT, out, s);
-  else
-    launch_gather<1>(batch, pitch, n_rows, ptr, col, wts, gT, out, s);
+  auto go = [&](auto v, auto g, auto p, int64_t ny) {
+    constexpr int V = decltype(v)::value, G = decltype(g)::value, P = decltype(p)::value;
+    launch_step(k_rows_gather<V, G, P>, dim3(unsigned(ceil_div(n_rows, kGatherWarps / P)), unsigned(ny)),
+                kGatherWarps * 32, 0, s, batch, pitch, n_rows, ptr, col, wts, gT, out);
+  };
+  // scratch that is not padded to a multiple of 4, or not aligned, is read in words
+  if (pitch % 4 == 0 && (reinterpret_cast<uintptr_t>(gT) & 15) == 0) pick_lanes<4>(pitch, n_rows, go);
+  else pick_lanes<1>(pitch, n_rows, go);
   BT_CHECK_LAUNCH("k_rows_gather");
   return BT_OK;
+}
+
+// ------------------------------------------------- forward, any activity --
+//
+// out = x @ W in whatever order is faster for this x, as counted on the device:
+// few nonzeros are pushed along their sources' out-edges with fp32 reductions
+// in L2, many are gathered over every post's in-edges from x transposed.
+
+// Whether the gather is the faster one: 8 + 4 batch bytes an edge at 14 TB/s
+// against 145 G reductions/s over nonzeros x mean out-degree (from about 4 % of
+// nonzeros at 32 samples and more, 40 % at one).
+__device__ __forceinline__ bool push_dense(const int32_t* ctl, int64_t n_in, int64_t pitch) {
+  const long long cnt = *reinterpret_cast<const volatile int32_t*>(ctl);
+  return cnt * 96 > n_in * (8 + 4 * (pitch > 8 ? pitch : 8));
+}
+
+// list[k] = the flat indices of x's nonzeros (order of arrival), ctl[0] their
+// count: 8 elements per thread, one atomic per block.
+__global__ void __launch_bounds__(256) k_compact(int64_t total, const float* __restrict__ x, int32_t* __restrict__ ctl,
+                                                 int32_t* __restrict__ list) {
+  __shared__ int s_warp[8], s_base;
+  const int lane = int(lane_id()), warp = int(threadIdx.x >> 5);
+  const int64_t base = int64_t(blockIdx.x) * 2048 + threadIdx.x;
+  uint32_t nz = 0;
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    if (base + u * 256 < total && __ldg(x + base + u * 256) != 0.0f) nz |= 1u << u;
+  const int cnt = __popc(nz);
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int w = 0; w < 8; ++w) {
+      const int c = s_warp[w];
+      s_warp[w] = sum;
+      sum += c;
+    }
+    s_base = sum ? atomicAdd(ctl, sum) : 0;
+  }
+  __syncthreads();
+  int at = s_base + s_warp[warp] + incl - cnt;
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    if (nz & (1u << u)) list[at++] = int32_t(base + u * 256);
+}
+
+// What the chosen path needs: x transposed (rows `pitch` apart, zeros past the
+// batch), or out cleared and, unless w_csr was given, the weights in CSR order.
+__global__ void __launch_bounds__(256) k_push_prepare(int64_t batch, int64_t n_in, int64_t n_out, int64_t pitch,
+                                                      int64_t nnz, const float* __restrict__ x,
+                                                      const int32_t* __restrict__ perm, const float* __restrict__ w,
+                                                      const int32_t* __restrict__ ctl, float* __restrict__ scratch,
+                                                      float* __restrict__ out) {
+  step_begin();
+  __shared__ float tile[32][33];
+  if (push_dense(ctl, n_in, pitch)) {
+    const int tx = int(threadIdx.x) & 31, ty = int(threadIdx.x) >> 5;
+    const int64_t nc = (n_in + 31) >> 5, nt = nc * ((pitch + 31) >> 5);
+    for (int64_t t = blockIdx.x; t < nt; t += gridDim.x) {
+      const int64_t c0 = t % nc * 32, r0 = t / nc * 32;
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 32; k += 8) {
+        const int64_t r = r0 + ty + k, c = c0 + tx;
+        if (c < n_in) tile[ty + k][tx] = r < batch ? __ldg(x + r * n_in + c) : 0.0f;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 32; k += 8) {
+        const int64_t c = c0 + ty + k, r = r0 + tx;
+        if (r < pitch && c < n_in) scratch[c * pitch + r] = tile[tx][ty + k];
+      }
+    }
+    return;
+  }
+  const int64_t tid = int64_t(blockIdx.x) * 256 + threadIdx.x, threads = int64_t(gridDim.x) * 256;
+  for (int64_t q = tid; q < batch * n_out; q += threads) out[q] = 0.0f;
+  if (perm) {
+    for (int64_t e = tid; e < nnz; e += 4 * threads) {
+      float v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = e + u * threads < nnz ? __ldg(w + __ldg(perm + e + u * threads)) : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (e + u * threads < nnz) scratch[e + u * threads] = v[u];
+    }
+  }
+}
+
+// The product by the chosen path.  The push streams a source's out-edges, 4 per
+// lane (two 128-bit loads when the CSR arrays allow, which the host checks).
+template <int V, int G, int P>
+__global__ void __launch_bounds__(kGatherWarps * 32) k_push_product(
+    int64_t batch, int64_t n_in, int64_t n_out, int64_t pitch, const int32_t* __restrict__ csr_ptr,
+    const uint32_t* __restrict__ csr_dst, const float* __restrict__ csr_w, const int32_t* __restrict__ csc_ptr,
+    const uint32_t* __restrict__ csc_src, const float* __restrict__ w, const float* __restrict__ x,
+    const int32_t* __restrict__ ctl, const int32_t* __restrict__ list, const float* __restrict__ xT,
+    float* __restrict__ out) {
+  step_begin();
+  if (push_dense(ctl, n_in, pitch)) {
+    rows_gather<V, G, P, true>(batch, pitch, n_out, csc_ptr, csc_src, w, xT, out);
+    return;
+  }
+  const int32_t count = *reinterpret_cast<const volatile int32_t*>(ctl);
+  const int lane = int(lane_id());
+  const int64_t blk = int64_t(blockIdx.y) * gridDim.x + blockIdx.x;
+  const int64_t warps = int64_t(gridDim.x) * gridDim.y * kGatherWarps;
+  for (int64_t it = blk * kGatherWarps + (threadIdx.x >> 5); it < count; it += warps) {
+    const int32_t flat = list[it];
+    const int64_t b = flat / n_in, j = flat % n_in;
+    const float val = __ldg(x + flat);
+    const int32_t beg = csr_ptr[j], end = csr_ptr[j + 1];
+    float* row = out + b * n_out;
+    for (int32_t g = (beg & ~3) + lane * 4; g < end; g += 128) {
+      const uint4 d4 = __ldg(reinterpret_cast<const uint4*>(csr_dst + g));
+      const float4 w4 = *reinterpret_cast<const float4*>(csr_w + g);
+      const uint32_t dd[4] = {d4.x, d4.y, d4.z, d4.w};
+      const float ww[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (g + q >= beg && g + q < end) atomicAdd(row + (dd[q] & kIdMask), ww[q] * val);
+    }
+  }
 }
 
 }  // namespace bt
@@ -198,4 +340,51 @@ extern "C" int bt_spmv_grad_input_pad(int64_t batch, int64_t n_in, int64_t n_out
                                       float* grad_x, float* work, void* stream) {
   return grad_input_t(batch, ceil_div(batch, 4) * 4, n_in, n_out, csr_ptr, csr_dst, csr_w, grad_out, grad_x, work,
                       stream);
+}
+
+// work: 8 control words, the list of nonzeros, then x transposed or the packed weights
+extern "C" int64_t bt_spmv_push_work_words(int64_t batch, int64_t n_in, int64_t padded) {
+  if (batch < 0 || n_in < 0 || padded < 0) return 0;
+  const int64_t pitch = ceil_div(batch, 4) * 4;
+  return 8 + ceil_div(batch * n_in, 4) * 4 + std::max(pitch * n_in, ceil_div(padded, 4) * 4);
+}
+
+extern "C" int bt_spmv_push(int64_t batch, int64_t n_in, int64_t n_out, int64_t nnz, const int32_t* csr_ptr,
+                            const uint32_t* csr_dst, const int32_t* csr_perm, const float* csr_w, const int32_t* csc_ptr,
+                            const uint32_t* csc_src, const float* w, const float* x, float* out, int32_t* work,
+                            void* stream) {
+  BT_CHECK_ARG(batch >= 0 && n_in >= 0 && n_out >= 0 && nnz >= 0, "negative size");
+  BT_CHECK_ARG(batch * n_in < (int64_t(1) << 31), "batch * n_in must be below 2^31");
+  if (batch == 0 || n_out == 0) return BT_OK;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  BT_CHECK_ARG(out, "null pointer");
+  if (n_in == 0 || nnz == 0) {
+    if (cudaMemsetAsync(out, 0, sizeof(float) * size_t(batch * n_out), s) != cudaSuccess)
+      return bt_set_error(BT_ERR_CUDA, "memset failed");
+    return BT_OK;
+  }
+  BT_CHECK_ARG(csr_ptr && csr_dst && (csr_perm || csr_w) && csc_ptr && csc_src && w && x && work, "null pointer");
+  BT_CHECK_ARG(((reinterpret_cast<uintptr_t>(csr_dst) | reinterpret_cast<uintptr_t>(csr_w) |
+                 reinterpret_cast<uintptr_t>(work)) & 15) == 0, "edge arrays and work must be 16-byte aligned");
+  const int64_t pitch = ceil_div(batch, 4) * 4, total = batch * n_in;
+  int32_t* list = work + 8;
+  float* scratch = reinterpret_cast<float*>(work + 8 + ceil_div(total, 4) * 4);
+  if (cudaMemsetAsync(work, 0, sizeof(int32_t) * 4, s) != cudaSuccess)
+    return bt_set_error(BT_ERR_CUDA, "memset failed");
+  k_compact<<<unsigned(ceil_div(total, 2048)), 256, 0, s>>>(total, x, work, list);
+  BT_CHECK_LAUNCH("k_compact");
+  const int64_t most = std::max(std::max(ceil_div(batch * n_out, 1024), ceil_div(nnz, 1024)),
+                                ceil_div(n_in, 32) * ceil_div(pitch, 32));
+  launch_step(k_push_prepare, dim3(unsigned(std::min<int64_t>(148 * 8, most))), 256, 0, s, batch, n_in, n_out, pitch, nnz,
+              x, csr_w ? nullptr : csr_perm, w, work, scratch, out);
+  BT_CHECK_LAUNCH("k_push_prepare");
+  const float* packed = csr_w ? csr_w : scratch;
+  pick_lanes<4>(pitch, n_out, [&](auto v, auto g, auto p, int64_t ny) {
+    constexpr int V = decltype(v)::value, G = decltype(g)::value, P = decltype(p)::value;
+    launch_step(k_push_product<V, G, P>, dim3(unsigned(ceil_div(n_out, kGatherWarps / P)), unsigned(ny)),
+                kGatherWarps * 32, 0, s, batch, n_in, n_out, pitch, csr_ptr, csr_dst, packed, csc_ptr, csc_src, w, x, work,
+                list, scratch, out);
+  });
+  BT_CHECK_LAUNCH("k_push_product");
+  return BT_OK;
 }

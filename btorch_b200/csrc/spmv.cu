@@ -23,7 +23,8 @@ __global__ void k_nonzero_bits(int64_t rows, int64_t cols, int64_t words, const 
   if (lane_id() == 0) bits[gw] = m;
 }
 
-// One warp per output neuron i; for every sample the warp walks i's in-edges
+// One warp per output neuron i and sample (grid.y: enough warps for the chip, the
+// rest of the samples in turn); the warp walks i's in-edges
 // (ascending source) 32 at a time, ballots the ones whose input is nonzero and
 // folds them in order with fmaf:  acc = fma(w, x, acc).  Zero inputs are
 // skipped, which does not change the value: acc is never -0 (it starts at +0
@@ -36,7 +37,7 @@ __global__ void k_spmv_gather(int64_t batch, int64_t n_in, int64_t n_out, int64_
   if (i >= n_out) return;
   const unsigned lane = lane_id();
   const int32_t beg = csc_ptr[i], end = csc_ptr[i + 1];
-  for (int64_t b = 0; b < batch; ++b) {
+  for (int64_t b = blockIdx.y; b < batch; b += gridDim.y) {
     const uint32_t* brow = bits + b * words;
     const float* xrow = x + b * n_in;
     float acc = 0.0f;
@@ -183,6 +184,14 @@ static inline int grid_for_warps(int64_t warps, int threads = 256) {
   return int(ceil_div(warps * 32, threads));
 }
 
+// Ordered gather: warps per output until about 64 per SM are in flight (one
+// warp walking 16 samples of 2000 outputs in turn leaves the chip idle).
+static inline dim3 gather_grid(int64_t n_out, int64_t batch) {
+  int64_t y = ceil_div(148 * 64, n_out);
+  if (y > batch) y = batch;
+  return dim3(unsigned(grid_for_warps(n_out)), unsigned(y < 1 ? 1 : y));
+}
+
 extern "C" int bt_spmv_gather(int64_t batch, int64_t n_in, int64_t n_out, const int32_t* csc_ptr,
                               const uint32_t* csc_src, const float* csc_w, const float* x, float* out,
                               uint32_t* bits, void* stream) {
@@ -196,7 +205,7 @@ extern "C" int bt_spmv_gather(int64_t batch, int64_t n_in, int64_t n_out, const 
     k_nonzero_bits<<<grid_for_warps(batch * words), 256, 0, s>>>(batch, n_in, words, x, bits);
     BT_CHECK_LAUNCH("k_nonzero_bits");
   }
-  k_spmv_gather<<<grid_for_warps(n_out), 256, 0, s>>>(batch, n_in, n_out, words, csc_ptr, csc_src, csc_w, x,
+  k_spmv_gather<<<gather_grid(n_out, batch), 256, 0, s>>>(batch, n_in, n_out, words, csc_ptr, csc_src, csc_w, x,
                                                        bits, out);
   BT_CHECK_LAUNCH("k_spmv_gather");
   return BT_OK;
@@ -326,7 +335,7 @@ extern "C" int bt_spmv_gather_noalloc(int64_t batch, int64_t n_in, int64_t n_out
     k_nonzero_bits<<<grid_for_warps(batch * words), 256, 0, s>>>(batch, n_in, words, x, bits);
     BT_CHECK_LAUNCH("k_nonzero_bits");
   }
-  k_spmv_gather<<<grid_for_warps(n_out), 256, 0, s>>>(batch, n_in, n_out, words, csc_ptr, csc_src, csc_w, x, bits,
+  k_spmv_gather<<<gather_grid(n_out, batch), 256, 0, s>>>(batch, n_in, n_out, words, csc_ptr, csc_src, csc_w, x, bits,
                                                        out);
   BT_CHECK_LAUNCH("k_spmv_gather");
   return BT_OK;

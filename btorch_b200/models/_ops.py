@@ -115,12 +115,18 @@ def pack_csr_weights(layout: SparseLayout, w_canonical: torch.Tensor) -> torch.T
     return out
 
 
+def csr_perm32(layout: SparseLayout) -> torch.Tensor:
+    """CSR position -> canonical index as int32 (built once per layout)."""
+    perm = getattr(layout, "_csr_perm32", None)
+    if perm is None:
+        perm = layout._csr_perm32 = layout.csr_perm.to(torch.int32)
+    return perm
+
+
 def pack_edges(layout: SparseLayout, w_canonical: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """The (post, weight) records of the CSR view (bt_engine_desc.csr_edges),
     padded like csr_dst."""
-    perm = getattr(layout, "csr_perm32", None)
-    if perm is None:
-        perm = layout.csr_perm32 = layout.csr_perm.to(torch.int32)
+    perm = csr_perm32(layout)
     if out is None:
         out = torch.empty(2 * layout.csr_dst.numel(), device=w_canonical.device, dtype=torch.int32)
     L.check(L.lib().bt_pack_edges(layout.nnz, layout.csr_dst.numel(), layout.csr_dst.data_ptr(), perm.data_ptr(),
@@ -144,12 +150,13 @@ def _spmv(direction: str, layout: SparseLayout, x: torch.Tensor, w_canon: torch.
                                     w_canon.data_ptr(), x.data_ptr(), out.data_ptr(), bits.data_ptr(), s)
         L.check(st, "bt_spmv_gather")
     else:
-        if w_csr is None:
-            w_csr = pack_csr_weights(layout, w_canon)
-        work = torch.empty(B * n_in + 2, device=dev, dtype=torch.int32)
-        st = L.lib().bt_spmv_scatter(B, n_in, layout.n_out, layout.csr_ptr.data_ptr(), layout.csr_dst.data_ptr(),
-                                     w_csr.data_ptr(), x.data_ptr(), out.data_ptr(), work.data_ptr(), s)
-        L.check(st, "bt_spmv_scatter")
+        padded = layout.csr_dst.numel()
+        work = torch.empty(L.lib().bt_spmv_push_work_words(B, n_in, padded), device=dev, dtype=torch.int32)
+        st = L.lib().bt_spmv_push(B, n_in, layout.n_out, layout.nnz, layout.csr_ptr.data_ptr(),
+                                  layout.csr_dst.data_ptr(), csr_perm32(layout).data_ptr(), L.ptr(w_csr),
+                                  layout.csc_ptr.data_ptr(), layout.csc_src.data_ptr(), w_canon.data_ptr(),
+                                  x.data_ptr(), out.data_ptr(), work.data_ptr(), s)
+        L.check(st, "bt_spmv_push")
     return out
 
 

@@ -125,6 +125,22 @@ BT_API int bt_spmv_scatter(int64_t batch, int64_t n_in, int64_t n_out,
                     const float* csr_w, const float* x, float* out,
                     int32_t* work, void* stream);
 
+/* The product in the order that is faster for this x, by the count of its
+ * nonzeros on the device: pushed as bt_spmv_scatter, or gathered over the CSC
+ * from x transposed (a fixed tree of fmaf chains per output, zero inputs
+ * skipped).  w: weights in canonical order; csr_w: the same in CSR order
+ * (padded like csr_dst), or NULL with csr_perm, which packs them when the push
+ * runs.  csr_dst padded to a multiple of 4.  `work`:
+ * bt_spmv_push_work_words(batch, n_in, length of csr_dst) int32 words, 16-byte
+ * aligned. */
+BT_API int64_t bt_spmv_push_work_words(int64_t batch, int64_t n_in, int64_t padded);
+BT_API int bt_spmv_push(int64_t batch, int64_t n_in, int64_t n_out, int64_t nnz,
+                    const int32_t* csr_ptr, const uint32_t* csr_dst,
+                    const int32_t* csr_perm, const float* csr_w,
+                    const int32_t* csc_ptr, const uint32_t* csc_src,
+                    const float* w, const float* x, float* out, int32_t* work,
+                    void* stream);
+
 /* Allocation-free bt_spmv_gather.  No counterpart in the reference: it exists
  * for callers that cannot allocate device memory when they need the product
  * (stream capture under a fixed memory plan, loops that must not take the
