@@ -11,6 +11,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent
@@ -42,25 +43,20 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         return LIB
     LIB_DIR.mkdir(parents=True, exist_ok=True)
     tmp = LIB.with_suffix(".so.tmp")
-    cmd = [
-        nvcc(),
-        *ARCH,
-        "-O3",
-        "-lineinfo",
-        "-std=c++17",
-        "-Xcompiler",
-        "-fPIC,-fvisibility=hidden",
-        "-shared",
-        "-cudart",
-        "static",
-        "-o",
-        str(tmp),
-        *[str(CSRC / s) for s in SOURCES],
-    ]
+    flags = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden"]
     if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-        print(" ".join(cmd))
-    subprocess.run(cmd, check=True, cwd=str(CSRC))
+        flags.insert(0, "-Xptxas=-v")
+        print(" ".join([nvcc(), *flags, *SOURCES]))
+    with tempfile.TemporaryDirectory() as d:
+        # one compiler per source (the template-heavy engines take minutes each)
+        objs = [str(Path(d) / (s + ".o")) for s in SOURCES]
+        procs = [subprocess.Popen([nvcc(), *flags, "-c", "-o", o, str(CSRC / s)], cwd=str(CSRC))
+                 for s, o in zip(SOURCES, objs)]
+        failed = [s for s, p in zip(SOURCES, procs) if p.wait() != 0]
+        if failed:
+            raise RuntimeError(f"nvcc failed on {', '.join(failed)}")
+        subprocess.run([nvcc(), *ARCH, "-shared", "-cudart", "static", "-Xcompiler", "-fPIC,-fvisibility=hidden", "-o",
+                        str(tmp), *objs], check=True, cwd=str(CSRC))
     os.replace(tmp, LIB)
     return LIB
 
