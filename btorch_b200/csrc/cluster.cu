@@ -176,7 +176,201 @@ struct SrcGroup<false> {
   }
 };
 
-template <int KIND, bool HARD, bool USE_REF, bool FAST, int IDS>
+// One arrival on this CTA's own barrier (release: its plain stores so far).
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  uint64_t state;
+  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 %0, [%1];" : "=l"(state) : "r"(smem_addr(bar)) : "memory");
+  (void)state;
+}
+
+// What the time loop of a warp that owns one item needs from the set-up.
+struct ClusterTile {
+  int B, Tp, Wd, words, w0, tile_n, NWv, R, Hc, H, rank, CL;
+  int64_t n, p0;
+  float *s_v, *s_psc, *s_ref, *s_gk, *s_w;
+  void* s_src;
+  uint32_t* s_bits;
+  int *s_gptr, *s_len, *s_deg;
+  uint64_t* s_mbar;
+  volatile int* dead;
+  int* dead_word;
+  uint32_t expect;
+  unsigned spin;
+};
+
+// The time loop when every (word, sample) item of a tile has a warp of its own
+// and every divisor is fast.  The item's state stays in registers, its
+// addresses advance by additions, and the warps wait for a step's words each by
+// itself: besides the other CTAs' bytes the barrier counts one arrival per own
+// warp, after its plain store, so no CTA-wide barrier is left in the loop.  The
+// ids and weights of the first rows are loaded before the wait, those of a
+// block's successor before its chain.  The general loop spends 470 of its 1200
+// instructions per warp and step outside the in-edge walk (16 rows: 2.26 us a
+// step, 96 rows 3.1), which is what this one shortens.
+template <int KIND, bool HARD, bool USE_REF, int IDS>
+__device__ __forceinline__ void cluster_one(const bt_engine_desc& d, const ClusterTile& t, cg::cluster_group& cluster) {
+  constexpr bool SRC16 = IDS == 0, DELAY = IDS == 2, ALIF = KIND == BT_NEURON_ALIF;
+  using G4 = typename SrcGroup<SRC16>::T;
+  constexpr int NG = kClRows / 4;
+  const int warp = int(threadIdx.x >> 5), lane = int(threadIdx.x & 31);
+  const int b = warp / t.NWv, w = warp - b * t.NWv;
+  const int l = w * 32 + lane, q = b * t.Tp + l;
+  const bool valid = l < t.tile_n;
+  const int steps = int(d.n_steps), len = t.s_len[b];
+  const int64_t cells = int64_t(t.B) * t.n;
+  const int64_t cell = int64_t(b) * t.n + t.p0 + (valid ? l : 0);
+  float P = t.s_psc[q], v = t.s_v[q], ref = t.s_ref[q], gk = t.s_gk[q];
+  const NeuronParams prm = load_params<KIND, USE_REF>(d.neuron, 0);
+  const float pc = d.psc_coef_s;
+  const Div dpt = make_div(d.psc_tau_s, d.psc_fast_div, d.psc_rcp);
+  const G4* srcg = reinterpret_cast<const G4*>(t.s_src) + lane;
+  const float4* wg = reinterpret_cast<const float4*>(t.s_w) + lane;
+  const int gb = t.s_gptr[w], ge = t.s_gptr[w + 1];
+  // published words: byte offset of this item's word in a copy, the copies' stride
+  const uint32_t off0 = uint32_t(b * t.Wd + t.w0 + w) * 4u, cstride = uint32_t(t.B * t.Wd) * 4u;
+  const bool remote = lane < t.CL && lane != t.rank;
+  const uint32_t rbits = remote ? cluster_addr(t.s_bits, lane) + off0 : 0u;
+  const uint32_t rbar = remote ? cluster_addr(t.s_mbar, lane) : 0u;
+  const float* xp = d.x ? d.x + cell : nullptr;
+  uint32_t* rp = d.raster ? d.raster + int64_t(b) * t.words + t.w0 + w : nullptr;
+  const bool traces = d.v_trace || d.psc_trace || d.ref_trace || d.gk_trace || d.spikes;
+  int64_t tix = cell;
+  int h_t = int(d.t0 % t.H);
+  const int deg = t.s_deg[l];
+  float x_ahead = (xp && valid && 0 < len) ? __ldcs(xp) : 0.0f;
+  int kc = 0, kp = t.Hc - 1;  // the copies of steps k and k - 1
+  for (int k = 0; k <= steps; ++k) {
+    G4 sn[NG];
+    float4 wn[NG];
+    if (gb < ge) {
+#pragma unroll
+      for (int j = 0; j < NG; ++j) {
+        sn[j] = srcg[(gb + j) * 32];
+        wn[j] = wg[(gb + j) * 32];
+      }
+    }
+    if (k > 0) {
+      // z_{k-1}: every CTA's words of step k - 1
+      uint64_t* bar = t.s_mbar + ((k - 1) & 1);
+      unsigned polls = 0;
+      while (!mbar_done(bar, uint32_t(((k - 1) >> 1) & 1))) {
+        if (*t.dead) break;  // a wait gave up somewhere
+        if (++polls > t.spin) {
+          if (lane == 0) {
+            *t.dead = 1;
+            if (d.tile_work) atomicCAS(d.tile_work + 2, 0, BT_ERR_TIMEOUT);
+            for (int r = 0; r < t.CL; ++r) *reinterpret_cast<volatile int*>(cluster.map_shared_rank(t.dead_word, r)) = 1;
+          }
+          break;
+        }
+      }
+      __syncwarp();
+      // armed for step k + 1 before this warp publishes step k, which every sender
+      // of step k + 1 has to have received
+      if (threadIdx.x == 0 && !*t.dead && k + 1 < steps) mbar_arm(bar, t.expect);
+      if (k - 1 < len) {
+        const char* base = reinterpret_cast<const char*>(t.s_bits) + uint32_t(b * t.Wd) * 4u;
+        const char* bits = base + uint32_t(kp) * cstride;
+        float g = 0.0f;
+        for (int gc = gb; gc < ge; gc += NG) {
+          uint32_t sr[kClRows];
+          float wv[kClRows];
+#pragma unroll
+          for (int j = 0; j < NG; ++j) {
+            SrcGroup<SRC16>::split(sn[j], sr + 4 * j);
+            wv[4 * j] = wn[j].x;
+            wv[4 * j + 1] = wn[j].y;
+            wv[4 * j + 2] = wn[j].z;
+            wv[4 * j + 3] = wn[j].w;
+          }
+          uint32_t bw[kClRows];
+#pragma unroll
+          for (int u = 0; u < kClRows; ++u) {
+            if constexpr (DELAY) {
+              int c = kp - int(sr[u] >> kClBinShift);  // the copy of step k - 1 - bin
+              c += c < 0 ? t.Hc : 0;
+              bw[u] = *reinterpret_cast<const uint32_t*>(base + uint32_t(c) * cstride + ((sr[u] >> 3) & 0x1fffcu));
+            } else {
+              bw[u] = *reinterpret_cast<const uint32_t*>(bits + ((sr[u] >> 3) & 0x1ffffffcu));
+            }
+          }
+          if (gc + NG < ge) {
+#pragma unroll
+            for (int j = 0; j < NG; ++j) {
+              sn[j] = srcg[(gc + NG + j) * 32];
+              wn[j] = wg[(gc + NG + j) * 32];
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < kClRows; ++u)
+            if (int(__funnelshift_l(bw[u], bw[u], sr[u])) < 0) g = add(g, wv[u]);
+        }
+        P = add(psc_decay_k<true>(pc, dpt, P), g);
+      }
+      if (d.psc_trace && valid) d.psc_trace[tix - cells] = P;
+      if (d.stats && b == 0) {
+        // union and edges over the samples of step k - 1
+        uint32_t any = 0u;
+        for (int bb = 0; bb < t.B; ++bb) any |= t.s_bits[(kp * t.B + bb) * t.Wd + t.w0 + w];
+        const bool on = valid && ((any >> lane) & 1u);
+        const unsigned un = __reduce_add_sync(0xffffffffu, on ? 1u : 0u);
+        const unsigned ed = __reduce_add_sync(0xffffffffu, on ? unsigned(deg) : 0u);
+        if (lane == 0 && un) {
+          unsigned long long* st = reinterpret_cast<unsigned long long*>(d.stats + int64_t(k - 1) * 4);
+          atomicAdd(st + 0, (unsigned long long)un);
+          if (ed) atomicAdd(st + 2, (unsigned long long)ed);
+        }
+      }
+    }
+    if (k == steps) break;  // only the synapse update of the last step
+    float s = 0.0f;
+    if (k < len) {
+      const float I = xp ? add(P, x_ahead) : P;
+      s = neuron_update<KIND, HARD, USE_REF, true, true>(prm, I, v, ref, gk).spike;
+    }
+    const uint32_t word = __ballot_sync(0xffffffffu, valid && s != 0.0f);
+    const uint32_t off = uint32_t(kc) * cstride;
+    if (lane == t.rank) {
+      *reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(t.s_bits) + off0 + off) = word;
+      // not once a wait gave up: the phase may never complete then (no arming
+      // arrival, no bytes), and an arrival beyond its count is a fault
+      if (!*t.dead) mbar_arrive(t.s_mbar + (k & 1));
+    } else if (remote && !*t.dead) {
+      st_async_word(rbits + off, word, rbar + uint32_t(k & 1) * 8u);
+    }
+    if (traces && valid) {
+      if (d.v_trace) d.v_trace[tix] = v;
+      if (USE_REF && d.ref_trace) d.ref_trace[tix] = ref;
+      if (ALIF && d.gk_trace) d.gk_trace[tix] = gk;
+      if (d.spikes) d.spikes[tix] = s;
+    }
+    tix += cells;
+    if (xp) {
+      xp += cells;
+      x_ahead = (k + 1 < steps && valid && k + 1 < len) ? __ldcs(xp) : 0.0f;
+    }
+    if (lane == 0) {
+      if (k + t.H >= steps) d.hist[(int64_t(h_t) * t.B + b) * t.words + t.w0 + w] = word;  // the last H steps
+      if (rp) *rp = word;
+    }
+    if (rp) rp += int64_t(t.B) * t.words;
+    if (d.stats) {
+      const unsigned ev = __reduce_add_sync(0xffffffffu, (valid && s != 0.0f) ? unsigned(deg) : 0u);
+      if (lane == 0 && ev)
+        atomicAdd(reinterpret_cast<unsigned long long*>(d.stats + int64_t(k) * 4) + 1, (unsigned long long)ev);
+    }
+    h_t = h_t + 1 == t.H ? 0 : h_t + 1;
+    kp = kc;
+    kc = kc + 1 == t.Hc ? 0 : kc + 1;
+  }
+  t.s_psc[q] = P;
+  t.s_v[q] = v;
+  t.s_ref[q] = ref;
+  t.s_gk[q] = gk;
+}
+
+// ONE: cluster_one's time loop (every item has a warp, fast divisors).
+template <int KIND, bool HARD, bool USE_REF, bool FAST, int IDS, bool ONE>
 __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_desc d) {
   constexpr bool SRC16 = IDS == 0, DELAY = IDS == 2;
   extern __shared__ __align__(16) unsigned char cl_smem[];
@@ -269,8 +463,9 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
   volatile int* dead = &s_dead;
   const uint32_t expect = uint32_t(4 * B * (words - NWv));
   if (threadIdx.x == 0) {
-    mbar_init(&s_mbar[0], 1);
-    mbar_init(&s_mbar[1], 1);
+    // ONE: own warps' arrivals beside the arming one
+    mbar_init(&s_mbar[0], ONE ? 1u + unsigned(NWv * B) : 1u);
+    mbar_init(&s_mbar[1], ONE ? 1u + unsigned(NWv * B) : 1u);
     mbar_init_fence();
     s_dead = 0;
     mbar_arm(&s_mbar[0], expect);
@@ -293,6 +488,13 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
   __syncthreads();
   if (!*dead) (void)mbar_done(&s_mbar[2], 0);
 
+  if constexpr (ONE) {
+    static_assert(FAST, "cluster_one takes scalar parameters with fast divisors");
+    const ClusterTile t{B,    Tp,  Wd,    words, w0,    tile_n, NWv,    R,     Hc,    H,     rank,   CL,    n,
+                        p0,   s_v, s_psc, s_ref, s_gk,  s_w,    s_src,  s_bits, s_gptr, s_len, s_deg,  s_mbar, dead,
+                        &s_dead, expect, spin};
+    if (warp < NWv * B) cluster_one<KIND, HARD, USE_REF, IDS>(d, t, cluster);
+  } else {
   const int items = NWv * B;  // (word, sample) pairs of this tile; item it = (b, w) = divmod(it, NWv)
   int h_t = int(d.t0 % H);
   // the drive of the warp's first item, loaded one step ahead (behind the barrier)
@@ -459,10 +661,13 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
     kp = kc;
     kc = kc + 1 == Hc ? 0 : kc + 1;
   }
+  }
   // every remote store into this CTA was waited for (the last iteration's
   // wait covers the last step); the barrier keeps every CTA resident until
   // all have left the loop, also when a wait gave up
   cluster.sync();
+  // words still under way when the others stopped waiting land before any CTA exits
+  if (*dead) __nanosleep(20000u);
   for (int q = threadIdx.x; q < B * Tp; q += T) {
     const int b = q / Tp, l = q - b * Tp;
     if (l >= tile_n) continue;
@@ -474,9 +679,9 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
   }
 }
 
-template <int KIND, bool HARD, bool USE_REF, bool FAST, int IDS>
+template <int KIND, bool HARD, bool USE_REF, bool FAST, int IDS, bool ONE>
 int cluster_launch(const bt_engine_desc& d, cudaStream_t s) {
-  void (*kern)(bt_engine_desc) = k_cluster_engine<KIND, HARD, USE_REF, FAST, IDS>;
+  void (*kern)(bt_engine_desc) = k_cluster_engine<KIND, HARD, USE_REF, FAST, IDS, ONE>;
   const int CL = d.n_tiles;
   const size_t smem = cluster_smem(d.n, d.batch, d.tile_posts, d.tile_rows, IDS == 0, cluster_copies(d.n_bins)).total;
   int dev = 0;
@@ -515,13 +720,22 @@ int cluster_launch(const bt_engine_desc& d, cudaStream_t s) {
 
 template <int KIND, bool HARD, bool USE_REF>
 int cluster_pick(const bt_engine_desc& d, bool fast, cudaStream_t s) {
-  switch (cluster_ids(d.n, d.n_bins)) {  // the encoding the packed ids were written in
+  const int ids = cluster_ids(d.n, d.n_bins);  // the encoding the packed ids were written in
+  // a warp per item: 16 warps at most
+  if (fast && int64_t(d.tile_posts / 32) * d.batch <= kClThreadsMax / 32)
+    return ids == 0   ? cluster_launch<KIND, HARD, USE_REF, true, 0, true>(d, s)
+           : ids == 1 ? cluster_launch<KIND, HARD, USE_REF, true, 1, true>(d, s)
+                      : cluster_launch<KIND, HARD, USE_REF, true, 2, true>(d, s);
+  switch (ids) {
     case 0:
-      return fast ? cluster_launch<KIND, HARD, USE_REF, true, 0>(d, s) : cluster_launch<KIND, HARD, USE_REF, false, 0>(d, s);
+      return fast ? cluster_launch<KIND, HARD, USE_REF, true, 0, false>(d, s)
+                  : cluster_launch<KIND, HARD, USE_REF, false, 0, false>(d, s);
     case 1:
-      return fast ? cluster_launch<KIND, HARD, USE_REF, true, 1>(d, s) : cluster_launch<KIND, HARD, USE_REF, false, 1>(d, s);
+      return fast ? cluster_launch<KIND, HARD, USE_REF, true, 1, false>(d, s)
+                  : cluster_launch<KIND, HARD, USE_REF, false, 1, false>(d, s);
     default:
-      return fast ? cluster_launch<KIND, HARD, USE_REF, true, 2>(d, s) : cluster_launch<KIND, HARD, USE_REF, false, 2>(d, s);
+      return fast ? cluster_launch<KIND, HARD, USE_REF, true, 2, false>(d, s)
+                  : cluster_launch<KIND, HARD, USE_REF, false, 2, false>(d, s);
   }
 }
 
