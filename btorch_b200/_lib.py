@@ -171,7 +171,8 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def stream_of(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    # the raw handle: torch.cuda.current_stream builds a Stream object (9 us a call)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def require_cuda(*tensors: torch.Tensor, what: str = "btorch_b200") -> torch.device:

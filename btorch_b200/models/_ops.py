@@ -325,9 +325,14 @@ def _desc_key(node, dt):
     sg = node.surrogate_function
     key = [float(dt), type(node), bool(node.hard_reset), bool(node._use_refractory),
            getattr(sg, "spiking", True), getattr(sg, "slope", None), getattr(sg, "damping_factor", None)]
+    params, buffers = node._parameters, node._buffers
     for name in _DESC_PARAMS:
-        t = getattr(node, name, None)
-        key.append((id(t), t.data_ptr(), _version(t), tuple(t.shape)) if torch.is_tensor(t) else t)
+        t = params.get(name)
+        if t is None:
+            t = buffers.get(name)
+        if t is None:
+            t = getattr(node, name, None)
+        key.append((id(t), t.data_ptr(), _version(t), t.shape) if isinstance(t, torch.Tensor) else t)
     return tuple(key)
 
 

@@ -17,6 +17,7 @@ from typing import Any
 
 import numpy as np
 import torch
+from torch.nn.modules import module as _module
 
 from .surrogate import Sigmoid
 
@@ -221,6 +222,12 @@ def _memory_var(rv: ResetValue, batch_size, **fmt) -> torch.Tensor:
     elif rv.value is None:
         return torch.empty(sizes, **fmt)
     else:
+        device = fmt.get("device")
+        if device is not None and torch.device(device).type != "cpu" and np.ndim(rv.value) == 0 \
+                and not (torch.is_tensor(rv.value) and rv.value.is_cuda):
+            # a scalar is filled in on the device (a copy from the host would wait for the stream)
+            t = torch.as_tensor(rv.value)
+            return torch.full(sizes, t.item(), dtype=fmt.get("dtype") or t.dtype, device=device)
         v = torch.as_tensor(rv.value, **fmt).detach().clone()
     if tuple(v.shape) != sizes:
         v = torch.broadcast_to(v, sizes).clone()
@@ -236,6 +243,16 @@ class MemoryModule(StepModule, torch.nn.Module):
         self._memories_rv: dict[str, ResetValue] = {}
         self._backend = "torch"
         self._step_mode = "s"
+
+    def __setattr__(self, name, value):
+        # a memory is rebound in every step: nn.Module's general path (parameter,
+        # module and buffer checks, then register_buffer again) costs 10 us each
+        rv = self.__dict__.get("_memories_rv")
+        if rv is not None and name in rv and type(value) is torch.Tensor and name in self._buffers \
+                and not _module._global_buffer_registration_hooks:
+            self._buffers[name] = value
+            return
+        super().__setattr__(name, value)
 
     @property
     def supported_backends(self):

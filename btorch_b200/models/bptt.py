@@ -527,10 +527,12 @@ def run(rnn, x: torch.Tensor, paths: dict):
         w_in = b_in = None
     C = checkpoint_chunk(rnn, T)
     kinds = frozenset(paths.values())
-    free = torch.cuda.mem_get_info(x.device)[0]
     need = _bytes_needed(T, B, n, C, kinds, isinstance(neuron, ALIF), neuron._use_refractory, inp is not None, c_in,
                          native_steps(rnn, B, n, syn.linear.direction(B)))
-    if need > MEMORY_FRACTION * free:
+    # (asking the driver for the free memory costs up to milliseconds: only for
+    # calls of a size that matters)
+    total = torch.cuda.get_device_properties(x.device).total_memory
+    if need > total // 64 and need > MEMORY_FRACTION * torch.cuda.mem_get_info(x.device)[0]:
         return None
     shape = v.shape
     v0 = v.reshape(B, n)

@@ -534,7 +534,10 @@ def run(plan: EnginePlan, rnn, x: torch.Tensor, sample_len: torch.Tensor | None 
         desc.spin_limit = int(getattr(rnn, "engine_spin_limit", 0))
     if mode == L.BT_MODE_CLUSTER:
         sl = slices_of(lay, dev)
-        shape = cluster_shape(n, B, lay.slices_ptr_host, choice.tile_posts, R)
+        shapes = lay.__dict__.setdefault("cluster_shapes", {})
+        if (B, choice.tile_posts, R) not in shapes:  # (by layout: its slices' rows)
+            shapes[B, choice.tile_posts, R] = cluster_shape(n, B, lay.slices_ptr_host, choice.tile_posts, R)
+        shape = shapes[B, choice.tile_posts, R]
         if shape is None:
             raise NotImplementedError("cluster mode: the network does not fit one cluster's shared memory")
         tp_c, P_c, rows_c = shape

@@ -42,13 +42,13 @@ class LIF(BaseNode):
         t = getattr(self, name)
         if t is None:
             raise RuntimeError(f"{type(self).__name__}.{name} is not initialised; call init_net_state() first.")
-        return t.reshape(-1, self.size)
+        return t if t.ndim == 2 and t.shape[1] == self.size else t.reshape(-1, self.size)
 
     def single_step_forward(self, x: torch.Tensor):
         dt = environ.get("dt")
         shape = self.v.shape if self.v is not None else None
         v2 = self._state2d("v")
-        x2 = x.reshape(-1, self.size)
+        x2 = x if x.ndim == 2 and x.shape[1] == self.size else x.reshape(-1, self.size)
         if x2.shape[0] != v2.shape[0]:
             x2 = torch.broadcast_to(x.reshape(-1, self.size), v2.shape)
         ref2 = self._state2d("refractory") if self._use_refractory else None
@@ -56,9 +56,13 @@ class LIF(BaseNode):
         if self.pre_spike_v:
             self.v_pre_spike = self.v.clone()
         spike, v_new, ref_new, gk_new = neuron_step(self, x2, v2, ref2, gk2, dt)
-        self.v = v_new.reshape(shape)
+        if v_new.shape != shape:
+            v_new, spike = v_new.reshape(shape), spike.reshape(shape)
+            ref_new = None if ref_new is None else ref_new.reshape(shape)
+            gk_new = None if gk_new is None else gk_new.reshape(shape)
+        self.v = v_new
         if ref_new is not None:
-            self.refractory = ref_new.reshape(shape)
+            self.refractory = ref_new
         if gk_new is not None:
-            self.g_k = gk_new.reshape(shape)
-        return spike.reshape(shape)
+            self.g_k = gk_new
+        return spike

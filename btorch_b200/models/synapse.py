@@ -76,8 +76,13 @@ class ExponentialPSC(BasePSC):
         coef, tau = self.coefficients(environ.get("dt"))
         wz = self._wz(z)
         shape = self.psc.shape
-        wz = torch.broadcast_to(wz, shape).reshape(-1, self.size)
-        self.psc = psc_step(self.psc.reshape(-1, self.size), wz, coef, tau).reshape(shape)
+        if wz.shape != shape:
+            wz = torch.broadcast_to(wz, shape)
+        psc = self.psc
+        if len(shape) != 2 or shape[1] != self.size:
+            wz, psc = wz.reshape(-1, self.size), psc.reshape(-1, self.size)
+        out = psc_step(psc, wz, coef, tau)
+        self.psc = out if out.shape == shape else out.reshape(shape)
         return self.psc
 
 
