@@ -59,6 +59,29 @@ __device__ __forceinline__ uint64_t l2_evict_last() {
   asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
+__device__ __forceinline__ uint64_t l2_evict_normal() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+// Loads that bring the whole 128-byte line into L2: what follows is read soon.
+__device__ __forceinline__ uint2 ld_nc_u2_line(const void* ptr, uint64_t pol) {
+  uint2 v;
+  asm("ld.global.nc.L2::cache_hint.L2::128B.v2.u32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(ptr), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_nc_u4_line(const void* ptr, uint64_t pol) {
+  uint4 v;
+  asm("ld.global.nc.L2::cache_hint.L2::128B.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(ptr), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ int32_t ld_nc_s32_line(const int32_t* ptr) {
+  int32_t v;
+  asm("ld.global.nc.L2::128B.s32 %0, [%1];" : "=r"(v) : "l"(ptr));
+  return v;
+}
 // Read-only (non-coherent) loads with an L2 policy; not volatile, so the
 // compiler may batch them ahead of their uses.
 __device__ __forceinline__ uint4 ld_nc_u4(const void* ptr, uint64_t pol) {

@@ -881,7 +881,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
   constexpr int kPerWarp = 32 / G;
   const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   const int n32 = int(n * n_rec(d));  // acc row stride; batch * n * C < 2^31 (checked on the host)
-  const uint64_t pol_stream = l2_evict_first(), pol_keep = l2_evict_last();
+  // (as k_eng_scatter_flat: lines with the following rows, for the next steps)
+  const uint64_t pol_edges = R > 1 ? l2_evict_normal() : l2_evict_first(), pol_keep = l2_evict_last();
   long long ev = 0, ed = 0;
   for (int64_t base = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kPerWarp; base < count;
        base += warps * kPerWarp) {
@@ -895,8 +896,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
       mrow = r.mask;
       flag = r.bin == d.bin_hi ? r.flag : nullptr;  // this set is not read again: clear it
       const int64_t row = int64_t(r.j) * R + r.bin;
-      beg = d.csr_ptr[row];
-      end = d.csr_ptr[row + 1];
+      beg = ld_nc_s32_line(d.csr_ptr + row);
+      end = ld_nc_s32_line(d.csr_ptr + row + 1);
     }
     // MS is the compile-time bound (1, 2, 4 or 8); the row holds ms words
     // (5..8 samples words above 128 samples run with MS = 8)
@@ -927,8 +928,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
         const int32_t gi = g0 + u * G * 4;
         if (gi < end) {
           // edges gi .. gi+3 as (post, weight) records: two 128-bit loads
-          const uint4 a = ld_nc_u4(d.csr_edges + 2 * int64_t(gi), pol_stream);
-          const uint4 b = ld_nc_u4(d.csr_edges + 2 * int64_t(gi) + 4, pol_stream);
+          const uint4 a = ld_nc_u4_line(d.csr_edges + 2 * int64_t(gi), pol_edges);
+          const uint4 b = ld_nc_u4_line(d.csr_edges + 2 * int64_t(gi) + 4, pol_edges);
           dq[u] = make_uint4(a.x, a.z, b.x, b.z);
           wq[u] = make_uint4(a.y, a.w, b.y, b.w);
         } else {
@@ -995,7 +996,9 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_fl
   const int lane = int(lane_id());
   const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   const int n32 = int(d.n * n_rec(d));  // acc row stride; batch * n * C < 2^31 (checked on the host)
-  const uint64_t pol_stream = l2_evict_first(), pol_keep = l2_evict_last();
+  // a neuron's rows are consecutive and read in consecutive steps: whole lines
+  // are brought in and kept for the next steps (one bin: read once, given up first)
+  const uint64_t pol_edges = R > 1 ? l2_evict_normal() : l2_evict_first(), pol_keep = l2_evict_last();
   long long ev = 0, ed = 0;
   // rows per warp and pass: an even share of the step's rows, 32 at most
   const int64_t share = (count + warps - 1) / warps;
@@ -1008,8 +1011,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_fl
     if (lane < rpw && it < count) {
       const ListedRow r = listed_row(d, si, ws0, s_off, planes, int32_t(it));
       const int64_t row = int64_t(r.j) * R + r.bin;
-      beg = d.csr_ptr[row];
-      len = d.csr_ptr[row + 1] - beg;
+      beg = ld_nc_s32_line(d.csr_ptr + row);
+      len = ld_nc_s32_line(d.csr_ptr + row + 1) - beg;
       int nsamp = 0;
 #pragma unroll
       for (int w = 0; w < MS; ++w) {
@@ -1062,7 +1065,7 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_fl
         wv[u] = 0.0f;
         if (e < total) {
           const int32_t g = rbeg + (e - rexcl);
-          const uint2 e = ld_nc_u2(d.csr_edges + 2 * int64_t(g), pol_stream);
+          const uint2 e = ld_nc_u2_line(d.csr_edges + 2 * int64_t(g), pol_edges);
           pp[u] = int(e.x & kIdMask);
           wv[u] = __uint_as_float(e.y);
         } else {
