@@ -361,6 +361,74 @@ __global__ void __launch_bounds__(kEngThreads) k_eng_neuron(bt_engine_desc d, in
   publish_spikes_ws(ws, i, b0, spiked);
 }
 
+// x / d for 4 values by a divisor of kind 1 or 2 (divk<true>, bit for bit): one
+// uniform branch on the kind and one on the rare cases for the four of them.  A
+// zero takes the fast path (its quotient is x r, sign included): silent synapses
+// and freshly reset neurons are in every warp, and the out-of-line path for one
+// lane costs the whole warp.
+__device__ __forceinline__ void divk4(const float (&x)[4], const Div& d, float (&out)[4]) {
+  if (d.kind == 1) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) out[q] = mul(x[q], d.r);
+    return;
+  }
+  bool rare = false;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float y = mul(x[q], d.r), ay = fabsf(y);
+    const float e = __fmaf_rn(-y, d.c, x[q]);
+    out[q] = x[q] == 0.0f ? y : __fmaf_rn(e, d.r, y);
+    rare |= !(ay >= 0x1p-100f && ay <= 0x1p100f) && x[q] != 0.0f;
+  }
+  if (rare) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) out[q] = div_recip(x[q], d.c, d.r);
+  }
+}
+
+// neuron_update<KIND, HARD, USE_REF, true, true> for 4 neurons with the same
+// (scalar) parameters, the same operations in the same order per neuron.
+template <int KIND, bool HARD, bool USE_REF>
+__device__ __forceinline__ void neuron_update4(const NeuronParams& pr, const float (&I)[4], float (&v)[4], float (&ref)[4],
+                                               float (&gk)[4], float (&s)[4]) {
+  float v1[4], t[4], a[4], b[4];
+  if (KIND == BT_NEURON_LIF) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) t[q] = -sub(v[q], pr.vr);
+    divk4(t, pr.d_tau, a);
+    divk4(I, pr.d_cm, b);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v1[q] = add(v[q], mul(pr.dt, add(a[q], b[q])));
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      t[q] = add(add(mul(pr.ngl, sub(v[q], pr.El)), mul(-gk[q], sub(v[q], pr.Ek))), I[q]);
+    divk4(t, pr.d_cm, a);  // derivative
+#pragma unroll
+    for (int q = 0; q < 4; ++q) t[q] = sub(pr.ngl, gk[q]);
+    divk4(t, pr.d_cm, b);  // linear
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float coef = div(expm1f(mul(pr.dt, b[q])), b[q]);
+      v1[q] = add(v[q], mul(coef, a[q]));
+      t[q] = -gk[q];
+    }
+    divk4(t, pr.d_tau_a, a);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) gk[q] = add(gk[q], mul(pr.cgk, a[q]));
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) t[q] = sub(v1[q], pr.vth);
+  divk4(t, pr.d_den, a);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    s[q] = (a[q] >= 0.0f && (!USE_REF || ref[q] == 0.0f)) ? 1.0f : 0.0f;
+    v[q] = HARD ? sub(v1[q], mul(sub(v1[q], pr.vr), s[q])) : sub(v1[q], mul(pr.den, s[q]));
+    if (KIND == BT_NEURON_ALIF) gk[q] = add(gk[q], mul(pr.dgk, s[q]));
+    if (USE_REF) ref[q] = relu_keep_nan(sub(add(ref[q], mul(s[q], pr.tau_ref)), pr.dt));
+  }
+}
+
 // Publish the spikes of one sample for the 4 neurons i0 .. i0 + 3 of this
 // thread (bit q of `nib`: neuron i0 + q), as publish_spikes_ws.  The warp's
 // 128 neurons share a sub-list when cap >= 128 (one atomic for the warp),
@@ -455,25 +523,45 @@ __global__ void __launch_bounds__(kVecThreads) k_eng_neuron_vec(bt_engine_desc d
   float acc[4] = {aq.x, aq.y, aq.z, aq.w}, P[4] = {pq.x, pq.y, pq.z, pq.w}, x[4] = {xq.x, xq.y, xq.z, xq.w};
   float v[4] = {vq.x, vq.y, vq.z, vq.w}, ref[4] = {rq.x, rq.y, rq.z, rq.w}, gk[4] = {gq.x, gq.y, gq.z, gq.w};
   float s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, stored[4];
-  NeuronParams prm = load_params<KIND, USE_REF>(d.neuron, valid ? i0 : 0);
-  float pc = d.psc_uniform ? d.psc_coef_s : 0.0f;
-  Div dpt = make_div(d.psc_uniform ? d.psc_tau_s : 1.0f, d.psc_uniform && d.psc_fast_div, d.psc_rcp);
+  if constexpr (FAST) {  // every parameter a scalar
+    const NeuronParams prm = load_params<KIND, USE_REF>(d.neuron, 0);
+    const Div dpt = make_div(d.psc_tau_s, d.psc_fast_div, d.psc_rcp);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = valid ? i0 + q : 0;
-    if (!FAST) {  // (FAST: every parameter a scalar)
+    for (int q = 0; q < 4; ++q) {
+      if (edge) P[q] = add(P[q], acc[q]);
+      stored[q] = P[q];
+    }
+    if (live) {
+      float I[4], t[4], a[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        I[q] = d.x ? add(P[q], x[q]) : P[q];
+        t[q] = -P[q];
+      }
+      neuron_update4<KIND, HARD, USE_REF>(prm, I, v, ref, gk, s);
+      divk4(t, dpt, a);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) stored[q] = add(P[q], mul(d.psc_coef_s, a[q]));
+    }
+  } else {
+    NeuronParams prm = load_params<KIND, USE_REF>(d.neuron, valid ? i0 : 0);
+    float pc = d.psc_uniform ? d.psc_coef_s : 0.0f;
+    Div dpt = make_div(d.psc_uniform ? d.psc_tau_s : 1.0f, d.psc_uniform && d.psc_fast_div, d.psc_rcp);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = valid ? i0 + q : 0;
       if (q > 0 && !d.neuron.uniform) prm = load_params<KIND, USE_REF>(d.neuron, i);
       if (!d.psc_uniform) {
         pc = ld(d.psc_coef, i);
         dpt = make_div(ld(d.psc_tau, i), false, 0.0f);
       }
-    }
-    if (edge) P[q] = add(P[q], acc[q]);
-    stored[q] = P[q];
-    if (live) {
-      const float I = d.x ? add(P[q], x[q]) : P[q];
-      s[q] = neuron_update<KIND, HARD, USE_REF, true, FAST>(prm, I, v[q], ref[q], gk[q]).spike;
-      stored[q] = psc_decay_k<FAST>(pc, dpt, P[q]);
+      if (edge) P[q] = add(P[q], acc[q]);
+      stored[q] = P[q];
+      if (live) {
+        const float I = d.x ? add(P[q], x[q]) : P[q];
+        s[q] = neuron_update<KIND, HARD, USE_REF, true, false>(prm, I, v[q], ref[q], gk[q]).spike;
+        stored[q] = psc_decay_k<false>(pc, dpt, P[q]);
+      }
     }
   }
   uint32_t nib = 0, own = 0;
