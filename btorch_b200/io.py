@@ -28,9 +28,11 @@ def _marker(nnz: int, shape, dims, dtype) -> tuple:
                                 "nnz": int(nnz)})
 
 
-def _encode(indices, data, shape, var_dims, var_name, dtype) -> dict[str, Any]:
+def _encode(indices, data, shape, var_dims, var_name, dtype, own: bool = False) -> dict[str, Any]:
+    """own: the index arrays are int32 and nobody else's (not copied again)."""
     sparse_dim = f"_btorch_sparse_idx_{var_name}"
-    out = {f"{var_name}_idx_{d}": ([sparse_dim], np.asarray(ix).astype(np.int32)) for d, ix in zip(var_dims, indices)}
+    out = {f"{var_name}_idx_{d}": ([sparse_dim], np.asarray(ix).astype(np.int32, copy=not own))
+           for d, ix in zip(var_dims, indices)}
     out[f"{var_name}_data"] = ([sparse_dim], np.asarray(data))
     out[var_name] = _marker(len(data), shape, var_dims, dtype)
     return out
@@ -72,8 +74,12 @@ def raster_to_sparse_repr(raster: torch.Tensor, n: int, var_name: str = "spikes"
     idx = torch.empty((3, max(nnz, 1)), dtype=torch.int32, device=dev)
     L.check(L.lib().bt_raster_coords(rows, B, n, bits.data_ptr(), offsets.data_ptr(), idx[0].data_ptr(),
                                      idx[1].data_ptr(), idx[2].data_ptr(), s), "bt_raster_coords")
-    ix = idx[:, :nnz].cpu().numpy()
-    return _encode((ix[0], ix[1], ix[2]), np.ones(nnz, dtype=dtype), (T, B, n), var_dims, var_name, dtype)
+    # one copy, into the arrays that are returned
+    ix = np.empty((3, nnz), dtype=np.int32)
+    if nnz:
+        torch.from_numpy(ix).copy_(idx)
+    return _encode((ix[0], ix[1], ix[2]), np.ones(nnz, dtype=dtype), (T, B, n), var_dims, var_name, dtype,
+                   own=True)
 
 
 def _values(entry):
