@@ -5,26 +5,49 @@
 
 namespace bt {
 
+constexpr int kHistWords = 8;  // words of a warp: 8 coalesced loads or stores in flight
+
+// Which (d, b) row and which words a warp owns; false past the end.
+__device__ __forceinline__ bool history_item(int64_t batch, int D, int64_t words, int64_t& d, int64_t& b, int64_t& w0) {
+  const int64_t gw = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t per = (words + kHistWords - 1) / kHistWords;
+  const int64_t rest = gw / per;
+  w0 = (gw - rest * per) * kHistWords;
+  d = rest / batch;
+  b = rest - d * batch;
+  return d < D;
+}
+
+__device__ __forceinline__ int64_t history_slot(const int64_t* cursor, int64_t advance, int64_t d, int D) {
+  if (!cursor) return d;
+  int64_t slot = (*cursor + advance - 1 - d) % D;
+  return slot < 0 ? slot + D : slot;
+}
+
 // ring[(t0 - 1 - d) mod H][b][w] = the spikes d steps ago, for d < D, from the
 // history memory hist[b][slot][n] (slot = (*cursor - 1 - d) mod D in circular
-// mode, d when cursor is NULL).  One warp per (d, b, word): coalesced loads, a
-// ballot per word.  Bound by the history's bytes.
+// mode, d when cursor is NULL).  A warp makes 8 words, a ballot each: bound by the
+// history's bytes (one word per warp took 219 us for 90 MB).
 __global__ void k_history_load(int64_t batch, int D, int64_t n, const float* __restrict__ hist,
                                const int64_t* __restrict__ cursor, int64_t t0, int H, uint32_t* __restrict__ ring) {
   const int64_t words = (n + 31) >> 5;
-  const int64_t gw = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t w = gw % words, rest = gw / words;
-  const int64_t b = rest % batch, d = rest / batch;
-  if (d >= D) return;
-  int64_t slot = d;
-  if (cursor) {
-    slot = (*cursor - 1 - d) % D;
-    if (slot < 0) slot += D;
+  int64_t d, b, w0;
+  if (!history_item(batch, D, words, d, b, w0)) return;  // whole warps
+  const int lane = int(lane_id());
+  const float* row = hist + (b * D + history_slot(cursor, 0, d, D)) * n;
+  float v[kHistWords];
+#pragma unroll
+  for (int u = 0; u < kHistWords; ++u) {
+    const int64_t i = (w0 + u) * 32 + lane;
+    v[u] = i < n ? __ldg(row + i) : 0.0f;
   }
-  const int64_t i = w * 32 + lane_id();
-  const bool on = i < n && __ldg(hist + (b * D + slot) * n + i) != 0.0f;
-  const uint32_t m = __ballot_sync(0xffffffffu, on);
-  if (lane_id() == 0) ring[(((t0 - 1 - d) % H) * batch + b) * words + w] = m;
+  uint32_t mine = 0u;
+#pragma unroll
+  for (int u = 0; u < kHistWords; ++u) {
+    const uint32_t m = __ballot_sync(0xffffffffu, v[u] != 0.0f);
+    if (lane == u) mine = m;
+  }
+  if (lane < kHistWords && w0 + lane < words) ring[(((t0 - 1 - d) % H) * batch + b) * words + w0 + lane] = mine;
 }
 
 // The reverse after `advance` steps: hist[b][slot(d)][n] = the spikes of step
@@ -32,18 +55,18 @@ __global__ void k_history_load(int64_t batch, int D, int64_t n, const float* __r
 __global__ void k_history_store(int64_t batch, int D, int64_t n, const uint32_t* __restrict__ ring, int64_t t_end, int H,
                                 const int64_t* __restrict__ cursor, int64_t advance, float* __restrict__ hist) {
   const int64_t words = (n + 31) >> 5;
-  const int64_t gw = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t w = gw % words, rest = gw / words;
-  const int64_t b = rest % batch, d = rest / batch;
-  if (d >= D) return;
-  int64_t slot = d;
-  if (cursor) {
-    slot = (*cursor + advance - 1 - d) % D;
-    if (slot < 0) slot += D;
+  int64_t d, b, w0;
+  if (!history_item(batch, D, words, d, b, w0)) return;
+  const int lane = int(lane_id());
+  float* row = hist + (b * D + history_slot(cursor, advance, d, D)) * n;
+  uint32_t mine = 0u;
+  if (lane < kHistWords && w0 + lane < words) mine = __ldg(ring + (((t_end - 1 - d) % H) * batch + b) * words + w0 + lane);
+#pragma unroll
+  for (int u = 0; u < kHistWords; ++u) {
+    const uint32_t m = __shfl_sync(0xffffffffu, mine, u);
+    const int64_t i = (w0 + u) * 32 + lane;
+    if (i < n) row[i] = float((m >> lane) & 1u);
   }
-  const uint32_t m = __ldg(ring + (((t_end - 1 - d) % H) * batch + b) * words + w);
-  const int64_t i = w * 32 + lane_id();
-  if (i < n) hist[(b * D + slot) * n + i] = float((m >> lane_id()) & 1u);
 }
 
 __global__ void k_cursor_advance(int64_t* cursor, int64_t advance, int D) { *cursor = (*cursor + advance) % D; }
@@ -76,7 +99,9 @@ int history_check(int64_t batch, int32_t D, int64_t n, int32_t H, int64_t t) {
   BT_CHECK_ARG(batch * n * D < (int64_t(1) << 38), "history too large");
   return BT_OK;
 }
-unsigned history_grid(int64_t batch, int32_t D, int64_t n) { return unsigned(ceil_div(batch * D * ((n + 31) / 32), 8)); }
+unsigned history_grid(int64_t batch, int32_t D, int64_t n) {
+  return unsigned(ceil_div(batch * D * ceil_div((n + 31) / 32, kHistWords), 8));
+}
 }  // namespace
 
 extern "C" int bt_history_load(int64_t batch, int32_t D, int64_t n, const float* hist, const int64_t* cursor, int64_t t0,
