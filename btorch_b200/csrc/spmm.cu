@@ -52,19 +52,23 @@ __device__ __forceinline__ FVec<V> ld_vec(const float* p) {
 }
 
 constexpr int kGatherWarps = 8;
+// Runs of gT in flight per lane (8: 4200 rows of 410 edges at batch 128 68 us, 88
+// with the 4 the compiler kept in flight; 64 registers, no spills).
+constexpr int kGatherUnroll = 8;
 
 // G lanes (a power of two) cover a block of G V samples at V samples each; the
 // S = 32 / G lane groups of a warp and the P warps of a row split its edges,
 // their partial sums meet in a butterfly and in shared memory (fixed order:
 // deterministic).  Without the lane groups a warp on 16 samples keeps 4 of its
 // lanes busy (18.9 us against 8.4 for 2000 rows of 100 edges); without the
-// warps per row 1000 rows leave the chip idle (45 against 21 us, 300 edges,
+// warps per row 1000 rows leave the chip idle (45 against 19 us, 300 edges,
 // batch 128).  Bound by the L1-miss path: 4 batch bytes an edge, 14 TB/s at
-// batch 128 (8192 rows of 410 edges: 119 us, 142 with a warp per row whose
+// batch 128 (8192 rows of 410 edges: 115 us, 142 with a warp per row whose
 // results went out as single words).  The CTA's rows are written through
 // shared memory, as runs of out[b].  Measured and slower: streaming gT
-// through shared memory in column tiles (195 us), and narrow sample blocks
-// with several rows per warp for reuse in L1 (150 us).
+// through shared memory in column tiles (195 us), narrow sample
+// blocks with several rows per warp for reuse in L1 (150 us), and CTAs of 32 rows in
+// step over windows of columns (138 us).
 // SKIP0: entries of gT that are zero add nothing, whatever the weight.
 template <int V, int G, int P, bool SKIP0>
 __device__ __forceinline__ void rows_gather(int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* __restrict__ ptr,
@@ -91,17 +95,25 @@ __device__ __forceinline__ void rows_gather(int64_t batch, int64_t pitch, int64_
       const float w = e < end ? __ldg(wts + e) : 0.0f;
       const int cnt = end - base < 32 ? end - base : 32;
       const int steps = (cnt + S - 1) / S;
-#pragma unroll 4
-      for (int q = 0; q < steps; ++q) {
-        const int k = q * S + grp;
-        const uint32_t cq = __shfl_sync(0xffffffffu, c, k);
-        const float wq = __shfl_sync(0xffffffffu, w, k);
-        if (in && k < cnt) {
-          const FVec<V> g = ld_vec<V>(gT + int64_t(cq) * pitch + bl);
+      // kGatherUnroll runs in flight per lane, then their chain
+      for (int q0 = 0; q0 < steps; q0 += kGatherUnroll) {
+        FVec<V> g[kGatherUnroll];
+        float wq[kGatherUnroll];
+#pragma unroll
+        for (int u = 0; u < kGatherUnroll; ++u) {
+          const int k = (q0 + u) * S + grp;
+          const uint32_t cq = __shfl_sync(0xffffffffu, c, k & 31);
+          wq[u] = __shfl_sync(0xffffffffu, w, k & 31);
+#pragma unroll
+          for (int v = 0; v < V; ++v) g[u].v[v] = 0.0f;
+          if (in && k < cnt) g[u] = ld_vec<V>(gT + int64_t(cq) * pitch + bl);
+          else wq[u] = 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < kGatherUnroll; ++u)
 #pragma unroll
           for (int v = 0; v < V; ++v)
-            if (!SKIP0 || g.v[v] != 0.0f) acc[v] = fmaf(wq, g.v[v], acc[v]);
-        }
+            if (!SKIP0 || g[u].v[v] != 0.0f) acc[v] = fmaf(wq[u], g[u].v[v], acc[v]);
       }
     }
 #pragma unroll
@@ -125,7 +137,7 @@ __device__ __forceinline__ void rows_gather(int64_t batch, int64_t pitch, int64_
 }
 
 template <int V, int G, int P>
-__global__ void __launch_bounds__(kGatherWarps * 32) k_rows_gather(int64_t batch, int64_t pitch, int64_t n_rows,
+__global__ void __launch_bounds__(kGatherWarps * 32, 4) k_rows_gather(int64_t batch, int64_t pitch, int64_t n_rows,
                                                                   const int32_t* __restrict__ ptr,
                                                                   const uint32_t* __restrict__ col,
                                                                   const float* __restrict__ wts,
@@ -273,7 +285,7 @@ __global__ void __launch_bounds__(256) k_push_prepare(int64_t batch, int64_t n_i
 // The product by the chosen path.  The push streams a source's out-edges, 4 per
 // lane (two 128-bit loads when the CSR arrays allow, which the host checks).
 template <int V, int G, int P>
-__global__ void __launch_bounds__(kGatherWarps * 32) k_push_product(
+__global__ void __launch_bounds__(kGatherWarps * 32, 3) k_push_product(
     int64_t batch, int64_t n_in, int64_t n_out, int64_t pitch, const int32_t* __restrict__ csr_ptr,
     const uint32_t* __restrict__ csr_dst, const float* __restrict__ csr_w, const int32_t* __restrict__ csc_ptr,
     const uint32_t* __restrict__ csc_src, const float* __restrict__ w, const float* __restrict__ x,
