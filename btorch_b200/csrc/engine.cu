@@ -731,11 +731,12 @@ __global__ void __launch_bounds__(kEngThreads) k_eng_neuron_rec(bt_engine_desc d
 // rows listed before counter c, s_off[planes * kSub] = rows of the step.  One
 // list over all planes lets every warp of the grid take its share of the rows
 // whatever bin they belong to.  *s_spk: spikes listed (one plane only).
+template <int T = kEngThreads>
 __device__ __forceinline__ void plane_offsets(const bt_engine_desc& d, const StepIdx& si, int planes, int32_t* s_off,
                                               int32_t* s_spk) {
-  __shared__ int32_t s_warp[kEngThreads / 32];
+  __shared__ int32_t s_warp[T / 32];
   const int Q = d.n_bins + 1, total = planes * kSub;
-  const int per = (total + kEngThreads - 1) / kEngThreads;
+  const int per = (total + T - 1) / T;
   const int c0 = int(threadIdx.x) * per, c1 = c0 + per < total ? c0 + per : total;
   int32_t sum = 0, spk = 0;
 #pragma unroll 4
@@ -761,13 +762,13 @@ __device__ __forceinline__ void plane_offsets(const bt_engine_desc& d, const Ste
   if (planes == 1 && spk) atomicAdd(s_spk, spk);
   int32_t run = incl - sum;
 #pragma unroll
-  for (int w = 0; w < kEngThreads / 32; ++w) run += w < warp ? s_warp[w] : 0;
+  for (int w = 0; w < T / 32; ++w) run += w < warp ? s_warp[w] : 0;
   for (int c = c0; c < c1; ++c) {
     const int32_t v = s_off[c];
     s_off[c] = run;
     run += v;
   }
-  if (threadIdx.x == kEngThreads - 1) s_off[total] = run;
+  if (threadIdx.x == T - 1) s_off[total] = run;
   __syncthreads();
 }
 
@@ -841,20 +842,19 @@ __device__ __forceinline__ void block_stats(const bt_engine_desc& d, int64_t k, 
 }
 
 // Dense delivery of one spike set (single delay bin): a block owns a slice of
-// 32 posts (lane = post); its 8 warps split the slice's rows of the sliced
+// 32 posts (lane = post); its W warps split the slice's rows of the sliced
 // in-edge view and accumulate, one 32-sample mask word per pass, into
 // per-warp shared-memory columns (no conflicts, no atomics); the block then
-// sums the 8 partial columns and stores the totals into acc with plain
-// stores (acc is zero on entry, each (sample, post) has one writer).  Used
+// sums the W partial columns and stores the totals into acc with plain
+// stores (acc is zero on entry, each (sample, post) has one writer).  s_acc:
+// W columns of 32 x 32 in shared memory, W the block's warps.  Used
 // for steps where most neurons spike in some sample, where per-event
 // reductions would cost more than reading every in-edge once.  The spike
 // set's masks and flags are then cleared by the last block to finish
 // (block-completion counter in ctrl[0]; no block waits for another).
-template <int MS>
-__device__ void scatter_dense(const bt_engine_desc& d, int64_t k, const ScatterScratch& ws, long long& ev,
+template <int MS, int W = kEngThreads / 32>
+__device__ void scatter_dense(const bt_engine_desc& d, const ScatterScratch& ws, float (*s_acc)[32][32], long long& ev,
                               long long& ed) {
-  constexpr int W = kEngThreads / 32;
-  __shared__ float s_acc[W][32][32];
   const int lane = int(lane_id()), wid = int(threadIdx.x >> 5);
   const int64_t n = d.n, B = d.batch;
   const int64_t nc = n * n_rec(d);  // acc columns (post * C + r)
@@ -960,7 +960,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
     int q = si.q_t - d.bin_lo;
     if (q < 0) q += R + 1;
     long long ev = 0, ed = 0;
-    scatter_dense<MS>(d, k, scatter_scratch(d, q), ev, ed);
+    __shared__ float s_acc[kEngThreads / 32][32][32];
+    scatter_dense<MS>(d, scatter_scratch(d, q), s_acc, ev, ed);
     if (d.stats) block_stats(d, k, ev, ed);
     return;
   }
@@ -1077,7 +1078,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_fl
     int q = si.q_t - d.bin_lo;
     if (q < 0) q += R + 1;
     long long ev = 0, ed = 0;
-    scatter_dense<MS>(d, k, scatter_scratch(d, q), ev, ed);
+    __shared__ float s_acc[kEngThreads / 32][32][32];
+    scatter_dense<MS>(d, scatter_scratch(d, q), s_acc, ev, ed);
     if (d.stats) block_stats(d, k, ev, ed);
     return;
   }
@@ -1176,6 +1178,143 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_fl
     }
   }
   if (d.stats) block_stats(d, k, ev, ed);
+}
+
+// Delivery sample by sample, summed in shared memory: a block takes one of
+// `parts` shares of a sample's spikes (listed from the step's bitmap), adds the
+// rows' edges into n accumulators in shared memory and then adds those, four at
+// a time, to the sample's row of acc.
+// k_eng_scatter is bound by its reductions in L2 (150 G/s over the device, 31
+// us for the 4.3M of a step at 8192 neurons, 410 edges a row, 128 samples, 1 %
+// spiking); additions in shared memory are about three times as fast and the
+// rows of acc are touched in whole lines: a training window of 100 such steps
+// 25.4 -> 22.9 ms.  One share per sample instead of two takes 25.2 ms: the
+// samples' spikes differ, and the busiest one is waited for; eight take 24.5,
+// each share pays its zeros and its n sums.  Shares of posts instead of spikes
+// read every edge in each of them (23.6 ms).
+// The spike set of the step, which the neuron launch still publishes (the dense
+// step reads it), is cleared whole.
+constexpr int kRowThreads = 512, kRowWarps = kRowThreads / 32, kRowList = 4096;
+constexpr int64_t kRowMaxN = 16384;  // accumulators and list of two blocks per SM: 160 KB
+template <int MS>
+__global__ void __launch_bounds__(kRowThreads, 2) k_eng_scatter_rows(bt_engine_desc d, StepIdx si, int parts) {
+  step_begin();
+  extern __shared__ __align__(16) float s_dyn[];  // [kRowList] row list, then accumulators or the dense step's columns
+  int32_t* s_list = reinterpret_cast<int32_t*>(s_dyn);
+  float* acc = s_dyn + kRowList;
+  const int bin = d.bin_lo, R = d.n_bins, n = int(d.n), B = int(d.batch);
+  int q = si.q_t - bin;
+  if (q < 0) q += R + 1;
+  const ScatterScratch ws = scatter_scratch(d, q);
+  clear_oldest_counts(d, si);
+  if (d.dense_rows > 0) {
+    __shared__ int32_t s_off[kSub + 1], s_spk;
+    plane_offsets<kRowThreads>(d, si, 1, s_off, &s_spk);
+    const int32_t count = s_off[kSub];
+    if (count >= d.dense_rows && s_spk >= kDenseSpikesPerRow * count) {  // grid-uniform
+      long long ev = 0, ed = 0;
+      scatter_dense<MS, kRowWarps>(d, ws, reinterpret_cast<float(*)[32][32]>(acc), ev, ed);
+      return;
+    }
+  }
+  const int tid = int(threadIdx.x), lane = int(lane_id()), wid = tid >> 5;
+  for (int i = int(blockIdx.x) * kRowThreads + tid; i < n * ws.ms; i += int(gridDim.x) * kRowThreads) ws.mask[i] = 0u;
+  for (int i = int(blockIdx.x) * kRowThreads + tid; i < n; i += int(gridDim.x) * kRowThreads) ws.flag[i] = 0;
+  const int b = int(blockIdx.x) / parts, part = int(blockIdx.x) - b * parts;
+  __shared__ int32_t s_warp[kRowWarps];
+  const int words = (n + 31) >> 5, per = (words + kRowThreads - 1) / kRowThreads;
+  const int w0 = tid * per < words ? tid * per : words, w1 = w0 + per < words ? w0 + per : words;
+  int h = si.h_t - bin;
+  if (h < 0) h += d.hist_len;
+  const uint32_t* bits = d.hist + (int64_t(h) * B + b) * words;
+  int cnt = 0;
+  for (int w = w0; w < w1; ++w) cnt += __popc(__ldcg(bits + w));
+  for (int i = tid; i < n; i += kRowThreads) acc[i] = 0.0f;
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_warp[wid] = incl;
+  __syncthreads();
+  const int wsum = lane < kRowWarps ? s_warp[lane] : 0;
+  const int total = int(__reduce_add_sync(0xffffffffu, unsigned(wsum)));
+  const int before = int(__reduce_add_sync(0xffffffffu, unsigned(lane < wid ? wsum : 0)));
+  const int first = before + incl - cnt;  // this thread's first spike among the sample's
+  // this block's share of the sample's spikes
+  const int own0 = int(int64_t(total) * part / parts), own1 = int(int64_t(total) * (part + 1) / parts);
+  if (own0 == own1) return;  // block-uniform
+  const uint64_t pol = l2_evict_normal();
+  for (int base = own0; base < own1; base += kRowList) {
+    const int rows = own1 - base < kRowList ? own1 - base : kRowList;
+    int at = first - base;
+    for (int w = w0; w < w1; ++w) {
+      uint32_t m = __ldcg(bits + w);
+      while (m) {
+        const int l = __ffs(m) - 1;
+        m &= m - 1;
+        if (at >= 0 && at < rows) s_list[at] = w * 32 + l;
+        ++at;
+      }
+    }
+    __syncthreads();
+    // warp w takes rows w, w + kRowWarps, ...: 32 row pointers at a time, one per lane
+    for (int r0 = wid; r0 < rows; r0 += kRowThreads) {
+      int32_t beg = 0, end = 0;
+      if (r0 + kRowWarps * lane < rows) {
+        const int64_t row = int64_t(s_list[r0 + kRowWarps * lane]) * R + bin;
+        beg = ld_nc_s32_line(d.csr_ptr + row);
+        end = ld_nc_s32_line(d.csr_ptr + row + 1);
+      }
+      const int nr = (rows - r0 + kRowWarps - 1) / kRowWarps;
+      for (int r = 0; r < (nr < 32 ? nr : 32); ++r) {
+        const int32_t rb = __shfl_sync(0xffffffffu, beg, r), re = __shfl_sync(0xffffffffu, end, r);
+        constexpr int U = 4;  // pairs of edges in flight per lane
+        for (int32_t e0 = (rb & ~1) + 2 * lane; e0 - 2 * lane < re; e0 += 64 * U) {
+          uint4 v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int32_t e = e0 + 64 * u;
+            v[u] = e < re ? ld_nc_u4_line(d.csr_edges + 2 * int64_t(e), pol) : make_uint4(0u, 0u, 0u, 0u);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int32_t e = e0 + 64 * u;
+            if (e >= rb && e < re) atomicAdd(acc + (v[u].x & kIdMask), __uint_as_float(v[u].y));
+            if (e + 1 < re) atomicAdd(acc + (v[u].z & kIdMask), __uint_as_float(v[u].w));
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // acc is zero on entry and holds a finite or infinite sum after it whatever the
+  // order of the shares; zeros add nothing
+  float* out = d.ring + int64_t(b) * n;
+  if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(d.ring) & 15) == 0) {
+    for (int i = 4 * tid; i < n; i += 4 * kRowThreads) {
+      const float4 f = *reinterpret_cast<const float4*>(acc + i);
+      if (f.x != 0.0f || f.y != 0.0f || f.z != 0.0f || f.w != 0.0f) atomicAdd(reinterpret_cast<float4*>(out + i), f);
+    }
+  } else {
+    for (int i = tid; i < n; i += kRowThreads)
+      if (acc[i] != 0.0f) atomicAdd(out + i, acc[i]);
+  }
+}
+
+// Shares per sample of k_eng_scatter_rows, 0 where k_eng_scatter is taken: one
+// delay bin, one channel, no statistics (they count the set's rows), long rows
+// (the 32-lane choice) and enough samples for two blocks per SM.  Windows of 40
+// training steps, k_eng_scatter against this one: 8192 neurons, batch 16: 3.76 /
+// 3.70 ms, 32: 4.81 / 4.37, 64: 6.95 / 6.49, 128: 10.9 / 9.9, 200: 17.5 / 15.9;
+// 2000 neurons, batch 64: 2.72 / 2.70, 4096, 128: 4.92 / 4.63, 16384, 128: 12.6 /
+// 12.0; but 30000, 64: 9.4 / 10.2 (zeros and sums of n per share).  A run driven
+// by given spikes needs them in the bitmap, which the vector neuron step writes.
+int row_parts(const bt_engine_desc& d, const float* z_given, bool vec, int sms) {
+  if (d.bin_lo != d.bin_hi || n_rec(d) != 1 || d.stats || d.scatter_lanes != 32 || (z_given && !vec)) return 0;
+  if (d.batch < 32 || d.n > kRowMaxN) return 0;
+  return int(std::max<int64_t>(2, 2 * sms / d.batch));
 }
 
 // psc_{t_end-1} = stored + acc; clears acc.
@@ -1903,12 +2042,27 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
     const bool vec = C == 1 && vec_neurons(d, z_given);
     const dim3 vgrid(unsigned(ceil_div(n, 4 * kVecThreads)), unsigned(d.batch));
     auto nvec = fast ? k_eng_neuron_vec<KIND, HARD, USE_REF, true> : k_eng_neuron_vec<KIND, HARD, USE_REF, false>;
+    const int parts = row_parts(d, z_given, vec, sms);
+    auto rows = ms == 1 ? k_eng_scatter_rows<1> : ms == 2 ? k_eng_scatter_rows<2> : ms <= 4 ? k_eng_scatter_rows<4>
+                                                                                             : k_eng_scatter_rows<8>;
+    const int64_t columns = d.dense_rows > 0 ? int64_t(kRowWarps) * 32 * 32 : 0;
+    const size_t rsmem = sizeof(float) * size_t(kRowList + std::max(n, columns));
+    if (parts) {
+      const void* kern = reinterpret_cast<const void*>(rows);
+      const size_t most = sizeof(float) * size_t(kRowList + kRowMaxN);
+      if (!launch_setup_known(kern, dev, most, 1)) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)) != cudaSuccess)
+          return bt_set_error(BT_ERR_CUDA, "shared memory request of %zu bytes refused", most);
+        launch_setup_add(kern, dev, most, 1);
+      }
+    }
     for (int64_t k = 0; k < d.n_steps; ++k) {
       const StepIdx si = step_idx(d.t0 + k, d.n_bins, d.hist_len);
       if (C > 1) launch_step(rec, rgrid, kEngThreads, 0, s, d, k, si);
       else if (vec) launch_step(nvec, vgrid, kVecThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
       else launch_step(neuron, grid, kEngThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
-      launch_step(scatter, dim3(sgrid), kEngThreads, ssmem, s, d, k, si);
+      if (parts) launch_step(rows, dim3(unsigned(d.batch * parts)), kRowThreads, rsmem, s, d, si, parts);
+      else launch_step(scatter, dim3(sgrid), kEngThreads, ssmem, s, d, k, si);
     }
     BT_CHECK_LAUNCH("k_eng_neuron/k_eng_scatter");
     if (d.n_steps > 0) {
