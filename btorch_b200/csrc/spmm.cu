@@ -368,6 +368,16 @@ extern "C" int bt_spmv_push(int64_t batch, int64_t n_in, int64_t n_out, int64_t 
   BT_CHECK_ARG(batch >= 0 && n_in >= 0 && n_out >= 0 && nnz >= 0, "negative size");
   BT_CHECK_ARG(batch * n_in < (int64_t(1) << 31), "batch * n_in must be below 2^31");
   if (batch == 0 || n_out == 0) return BT_OK;
+  // sample blocks are the grid's y (below 65536): larger batches go in slabs, one
+  // after the other through the same scratch
+  constexpr int64_t kSlab = int64_t(1) << 22;
+  if (batch > kSlab) {
+    for (int64_t b0 = 0; b0 < batch; b0 += kSlab)
+      if (int st = bt_spmv_push(std::min(kSlab, batch - b0), n_in, n_out, nnz, csr_ptr, csr_dst, csr_perm, csr_w, csc_ptr,
+                                csc_src, w, x ? x + b0 * n_in : nullptr, out ? out + b0 * n_out : nullptr, work, stream))
+        return st;
+    return BT_OK;
+  }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BT_CHECK_ARG(out, "null pointer");
   if (n_in == 0 || nnz == 0) {

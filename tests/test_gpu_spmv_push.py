@@ -62,3 +62,16 @@ def test_ordered_gather_samples_over_the_grid(batch, n_out):
     whole = _ops._spmv("gather", lay, x, wd, None)
     rows = torch.cat([_ops._spmv("gather", lay, x[b:b + 1].contiguous(), wd, None) for b in range(batch)])
     assert torch.equal(whole, rows)
+
+
+@pytest.mark.parametrize("activity", [0.02, 1.0])
+def test_push_batches_beyond_the_grid(activity):
+    """More samples than sample blocks fit the grid's y: dyadic weights, exact in any order."""
+    batch, n_in, n_out = (1 << 23) + 5, 3, 2
+    m = SparseConn.from_canonical(np.array([0, 0, 1, 1]), np.array([0, 2, 1, 2]),
+                                  np.array([0.5, -2.0, 1.0, 0.25], np.float32), (n_in, n_out), enforce_dale=False).to(DEV)
+    x = (torch.rand((batch, n_in), device=DEV) < activity).float()
+    got = _ops._spmv("scatter", m.layout(DEV), x, m.magnitude.detach(), None)
+    dense = torch.tensor([[0.5, 0.0], [0.0, 1.0], [-2.0, 0.25]], device=DEV)
+    want = x[:, :1] * dense[0] + x[:, 1:2] * dense[1] + x[:, 2:] * dense[2]
+    assert torch.equal(got, want)
