@@ -22,7 +22,11 @@ class SparseLayout:
 
     n_in = n_pre * n_bins presynaptic rows (delay-expanded), n_out = posts.
     Edge arrays of the CSR view are padded to a multiple of 4 entries (+4) so
-    that 128-bit vector loads never leave the allocation."""
+    that 128-bit vector loads never leave the allocation.
+
+    Every array comes from the host builder and reaches the device in `to`,
+    whose copies are complete when it returns: a layout may be read on any
+    stream.  Nothing is derived from it later on a caller's stream and kept."""
 
     n_pre: int
     n_bins: int
@@ -32,7 +36,7 @@ class SparseLayout:
     csc_src: torch.Tensor   # int32 (uint32 bits) [nnz]: pre | bin << 25
     csr_ptr: torch.Tensor   # int32 [n_pre + 1]
     csr_dst: torch.Tensor   # int32 (uint32 bits) [pad4(nnz)]: post | bin << 25
-    csr_perm: torch.Tensor  # int64 [nnz]: CSR position -> canonical index
+    csr_perm: torch.Tensor  # int32 [nnz]: CSR position -> canonical index
 
     @property
     def n_in(self) -> int:
@@ -67,7 +71,7 @@ def build_layout(indices: torch.Tensor, n_pre: int, n_out: int, n_bins: int = 1)
     as_t = lambda a: torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a)  # noqa: E731
     return SparseLayout(n_pre=n_pre, n_bins=n_bins, n_out=n_out, nnz=nnz, csc_ptr=as_t(csc_ptr),
                         csc_src=as_t(csc_src[:nnz].copy()), csr_ptr=as_t(csr_ptr), csr_dst=as_t(csr_dst),
-                        csr_perm=torch.from_numpy(csr_perm[:nnz].astype(np.int64)))
+                        csr_perm=torch.from_numpy(csr_perm[:nnz].copy()))
 
 
 @dataclass
@@ -115,18 +119,10 @@ def pack_csr_weights(layout: SparseLayout, w_canonical: torch.Tensor) -> torch.T
     return out
 
 
-def csr_perm32(layout: SparseLayout) -> torch.Tensor:
-    """CSR position -> canonical index as int32 (built once per layout)."""
-    perm = getattr(layout, "_csr_perm32", None)
-    if perm is None:
-        perm = layout._csr_perm32 = layout.csr_perm.to(torch.int32)
-    return perm
-
-
 def pack_edges(layout: SparseLayout, w_canonical: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """The (post, weight) records of the CSR view (bt_engine_desc.csr_edges),
     padded like csr_dst."""
-    perm = csr_perm32(layout)
+    perm = layout.csr_perm.to(torch.int32)  # (SparseLayout's own is)
     if out is None:
         out = torch.empty(2 * layout.csr_dst.numel(), device=w_canonical.device, dtype=torch.int32)
     L.check(L.lib().bt_pack_edges(layout.nnz, layout.csr_dst.numel(), layout.csr_dst.data_ptr(), perm.data_ptr(),
@@ -153,7 +149,7 @@ def _spmv(direction: str, layout: SparseLayout, x: torch.Tensor, w_canon: torch.
         padded = layout.csr_dst.numel()
         work = torch.empty(L.lib().bt_spmv_push_work_words(B, n_in, padded), device=dev, dtype=torch.int32)
         st = L.lib().bt_spmv_push(B, n_in, layout.n_out, layout.nnz, layout.csr_ptr.data_ptr(),
-                                  layout.csr_dst.data_ptr(), csr_perm32(layout).data_ptr(), L.ptr(w_csr),
+                                  layout.csr_dst.data_ptr(), layout.csr_perm.data_ptr(), L.ptr(w_csr),
                                   layout.csc_ptr.data_ptr(), layout.csc_src.data_ptr(), w_canon.data_ptr(),
                                   x.data_ptr(), out.data_ptr(), work.data_ptr(), s)
         L.check(st, "bt_spmv_push")
