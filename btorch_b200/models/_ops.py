@@ -13,6 +13,35 @@ import torch
 
 from .. import _lib as L
 
+# ------------------------------------------------- arrays kept across calls --
+
+
+class Kept:
+    """Device arrays formed from a module's tensors on one stream and kept for
+    later calls: `get` returns them once the current stream has been told to
+    wait for the stream that formed them.  Not for use while a stream is being
+    captured (`keepable`): what a capture records has not run, and a replay
+    must not depend on memory that the keeper may replace."""
+
+    def __init__(self, key, arrays, device):
+        self.key, self.arrays, self.device = key, tuple(arrays), device
+        self.stream = L.stream_of(device)
+        self.event = torch.cuda.Event()
+        self.event.record(torch.cuda.current_stream(device))
+
+    def get(self):
+        if L.stream_of(self.device) != self.stream:
+            cur = torch.cuda.current_stream(self.device)
+            cur.wait_event(self.event)
+            for t in self.arrays:
+                t.record_stream(cur)  # (the keeper may let go of it while this stream still reads)
+        return self.arrays
+
+
+def keepable() -> bool:
+    return not torch.cuda.is_current_stream_capturing()
+
+
 # ----------------------------------------------------------------- layout --
 
 
@@ -199,11 +228,13 @@ def _csr_weights_cached(layout, w):
     tensor object and version: a SparseConn's weight is its magnitude
     parameter, the same tensor in every step of a window until the optimizer
     updates it (weak reference, so a new tensor at a reused address misses)."""
+    if not keepable():
+        return pack_csr_weights(layout, w.detach())
     hit = getattr(layout, "_w_csr_cache", None)
-    if hit is not None and hit[0]() is w and hit[1] == (w.data_ptr(), _version(w)):
-        return hit[2]
+    if hit is not None and hit[0]() is w and hit[1].key == (w.data_ptr(), _version(w)):
+        return hit[1].get()[0]
     packed = pack_csr_weights(layout, w.detach())
-    layout._w_csr_cache = (weakref.ref(w), (w.data_ptr(), _version(w)), packed)
+    layout._w_csr_cache = (weakref.ref(w), Kept((w.data_ptr(), _version(w)), (packed,), w.device))
     return packed
 
 
@@ -343,9 +374,16 @@ def neuron_desc(node, dt: float):
     key = _desc_key(node, dt)
     hit = node.__dict__.get("_bt_neuron_desc")
     if hit is not None and hit[0] == key:
+        if hit[3] is not None and keepable():
+            hit[3].get()
         return hit[1], hit[2]
     d, keep = _build_neuron_desc(node, dt)
-    node.__dict__["_bt_neuron_desc"] = (key, d, keep)
+    own = {t.data_ptr() for t in (*node._parameters.values(), *node._buffers.values()) if t is not None}
+    formed = [t for t in keep if t.is_cuda and t.data_ptr() not in own]
+    if not formed:  # every array is a parameter's own memory
+        node.__dict__["_bt_neuron_desc"] = (key, d, keep, None)
+    elif keepable():
+        node.__dict__["_bt_neuron_desc"] = (key, d, keep, Kept(key, formed, formed[0].device))
     return d, keep
 
 

@@ -286,7 +286,9 @@ def tile_offsets(lay, edges: torch.Tensor, tp: int, P: int, dev) -> torch.Tensor
         off = torch.empty((rows, P + 1), device=dev, dtype=torch.int32)
         L.check(L.lib().bt_tile_offsets(rows, lay.csr_ptr.data_ptr(), edges.data_ptr(), tp, P, off.data_ptr(),
                                         L.stream_of(dev)), "bt_tile_offsets")
-        cache[(tp, P)] = off
+        if _ops.keepable():
+            torch.cuda.current_stream(dev).synchronize()  # complete for every stream that reads it from now on
+            cache[(tp, P)] = off
     return off
 
 
@@ -546,12 +548,13 @@ def run(plan: EnginePlan, rnn, x: torch.Tensor, sample_len: torch.Tensor | None 
         # effective weight's inputs) changed: in place (version) or replaced
         key = (tp_c, P_c, rows_c, R, str(dev),
                tuple((t.data_ptr(), t._version) for t in [*conn.parameters(), *conn.buffers()]))
-        cached = getattr(conn, "_cluster_packed", None)
-        if cached is not None and cached[0] == key:
-            cl_w, cl_src = cached[1], cached[2]
+        cached = getattr(conn, "_cluster_packed", None) if _ops.keepable() else None
+        if cached is not None and cached.key == key:
+            cl_w, cl_src = cached.get()
         else:
             cl_w, cl_src = cluster_pack(sl, pack_slice_weights(sl, w), index, n, R)
-            conn._cluster_packed = (key, cl_w, cl_src)
+            if _ops.keepable():
+                conn._cluster_packed = _ops.Kept(key, (cl_w, cl_src), dev)
         cl_w, cl_src = static("cl_w", cl_w), static("cl_src", cl_src)
         tile_ws = alloc("tile_work", (32,), torch.int32, zero=True)  # word 2: status (a wait that gave up)
         keep += [cl_w, cl_src, gptr, tile_ws]
