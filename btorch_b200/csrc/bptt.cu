@@ -230,7 +230,8 @@ extern "C" int bt_bptt_backward(const bt_bptt_desc* d, void* stream) {
     a.g_I = d->G_I + t * per;
     a.next_psc = t > 0 ? d->G_psc + (t - 1) * per : d->cur_psc;
     a.next_T = t > 0 ? d->gT : nullptr;
-    launch_step(kern, grid, 256, 0, s, nd, d->psc_coef, d->psc_tau, B, pitch, n, int(d->detach_reset), a);
+    if (launch_step(kern, grid, 256, 0, s, nd, d->psc_coef, d->psc_tau, B, pitch, n, int(d->detach_reset), a) != cudaSuccess)
+      break;
   }
   BT_CHECK_LAUNCH("k_bptt_step");
   return BT_OK;

@@ -945,7 +945,7 @@ __device__ void scatter_dense(const bt_engine_desc& d, const ScatterScratch& ws,
 template <int G, int MS>
 __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt_engine_desc d, int64_t k, StepIdx si) {
   step_begin();
-  extern __shared__ int32_t s_off[];  // [planes * kSub + 1]
+  extern __shared__ __align__(16) int32_t s_off[];  // [planes * kSub + 1], or the dense step's columns
   const int64_t n = d.n;
   const int R = d.n_bins, planes = d.bin_hi - d.bin_lo + 1;
   const ScatterScratch ws0 = scatter_scratch(d, 0);
@@ -960,8 +960,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
     int q = si.q_t - d.bin_lo;
     if (q < 0) q += R + 1;
     long long ev = 0, ed = 0;
-    __shared__ float s_acc[kEngThreads / 32][32][32];
-    scatter_dense<MS>(d, scatter_scratch(d, q), s_acc, ev, ed);
+    __syncthreads();  // the offsets have been read: their memory takes the columns
+    scatter_dense<MS>(d, scatter_scratch(d, q), reinterpret_cast<float(*)[32][32]>(s_off), ev, ed);
     if (d.stats) block_stats(d, k, ev, ed);
     return;
   }
@@ -1064,7 +1064,7 @@ template <int MS>
 __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_flat(bt_engine_desc d, int64_t k,
                                                                               StepIdx si) {
   step_begin();
-  extern __shared__ int32_t s_off[];  // [planes * kSub + 1]
+  extern __shared__ __align__(16) int32_t s_off[];  // [planes * kSub + 1], or the dense step's columns
   const int R = d.n_bins, planes = d.bin_hi - d.bin_lo + 1;
   const ScatterScratch ws0 = scatter_scratch(d, 0);
   __shared__ int32_t s_spk;
@@ -1078,8 +1078,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_fl
     int q = si.q_t - d.bin_lo;
     if (q < 0) q += R + 1;
     long long ev = 0, ed = 0;
-    __shared__ float s_acc[kEngThreads / 32][32][32];
-    scatter_dense<MS>(d, scatter_scratch(d, q), s_acc, ev, ed);
+    __syncthreads();  // the offsets have been read: their memory takes the columns
+    scatter_dense<MS>(d, scatter_scratch(d, q), reinterpret_cast<float(*)[32][32]>(s_off), ev, ed);
     if (d.stats) block_stats(d, k, ev, ed);
     return;
   }
@@ -2016,7 +2016,10 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
     const int64_t rows_per_block = d.scatter_lanes == 1 ? 64 : d.scatter_lanes == 8 ? kEngThreads / 8 : kEngThreads / 32;
     const int64_t wave = int64_t(sms) * (ms <= 4 ? 4 : 3);
     const unsigned sgrid = unsigned(std::max<int64_t>(1, std::min(wave, ceil_div(n * planes, rows_per_block))));
-    const size_t ssmem = sizeof(int32_t) * size_t(planes * kSub + 1);
+    // the offsets of all planes, or the columns of a dense step, which has one plane:
+    // at most 33 KB (128 bins), within the 48 KB that need no attribute
+    const size_t ssmem = std::max(sizeof(int32_t) * size_t(planes * kSub + 1),
+                                  d.dense_rows > 0 ? sizeof(float) * (kEngThreads / 32) * 32 * 32 : size_t(0));
     // every divisor a power of two or a verified reciprocal: no IEEE division compiled in
     const bool fast = fast_divisors(d, KIND);
     auto neuron = fast ? (S == 1 ? k_eng_neuron<KIND, HARD, USE_REF, 1, true>
@@ -2058,11 +2061,14 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
     }
     for (int64_t k = 0; k < d.n_steps; ++k) {
       const StepIdx si = step_idx(d.t0 + k, d.n_bins, d.hist_len);
-      if (C > 1) launch_step(rec, rgrid, kEngThreads, 0, s, d, k, si);
-      else if (vec) launch_step(nvec, vgrid, kVecThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
-      else launch_step(neuron, grid, kEngThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
-      if (parts) launch_step(rows, dim3(unsigned(d.batch * parts)), kRowThreads, rsmem, s, d, si, parts);
-      else launch_step(scatter, dim3(sgrid), kEngThreads, ssmem, s, d, k, si);
+      // nothing runs on after a refused launch: the state would move on without its input
+      cudaError_t e = C > 1 ? launch_step(rec, rgrid, kEngThreads, 0, s, d, k, si)
+                      : vec ? launch_step(nvec, vgrid, kVecThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given)
+                            : launch_step(neuron, grid, kEngThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
+      if (e == cudaSuccess)
+        e = parts ? launch_step(rows, dim3(unsigned(d.batch * parts)), kRowThreads, rsmem, s, d, si, parts)
+                  : launch_step(scatter, dim3(sgrid), kEngThreads, ssmem, s, d, k, si);
+      if (e != cudaSuccess) break;
     }
     BT_CHECK_LAUNCH("k_eng_neuron/k_eng_scatter");
     if (d.n_steps > 0) {
