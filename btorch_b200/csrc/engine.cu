@@ -942,10 +942,11 @@ __device__ void scatter_dense(const bt_engine_desc& d, const ScatterScratch& ws,
 // Launch bounds: at least 4 (MS <= 4) or 3 resident blocks per SM, which
 // leaves ptxas 64 / 85 registers -- without a bound its occupancy heuristic
 // has settled on 48 registers and spilled the reduction loop.
+constexpr size_t kScatterStatic = 33 * 1024;  // at least the static shared memory of k_eng_scatter and k_eng_scatter_flat
 template <int G, int MS>
 __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt_engine_desc d, int64_t k, StepIdx si) {
   step_begin();
-  extern __shared__ __align__(16) int32_t s_off[];  // [planes * kSub + 1], or the dense step's columns
+  extern __shared__ int32_t s_off[];  // [planes * kSub + 1]
   const int64_t n = d.n;
   const int R = d.n_bins, planes = d.bin_hi - d.bin_lo + 1;
   const ScatterScratch ws0 = scatter_scratch(d, 0);
@@ -960,8 +961,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter(bt
     int q = si.q_t - d.bin_lo;
     if (q < 0) q += R + 1;
     long long ev = 0, ed = 0;
-    __syncthreads();  // the offsets have been read: their memory takes the columns
-    scatter_dense<MS>(d, scatter_scratch(d, q), reinterpret_cast<float(*)[32][32]>(s_off), ev, ed);
+    __shared__ float s_acc[kEngThreads / 32][32][32];  // (beside the offsets: overlaid on them, 1.4 % slower at 20 bins)
+    scatter_dense<MS>(d, scatter_scratch(d, q), s_acc, ev, ed);
     if (d.stats) block_stats(d, k, ev, ed);
     return;
   }
@@ -1064,7 +1065,7 @@ template <int MS>
 __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_flat(bt_engine_desc d, int64_t k,
                                                                               StepIdx si) {
   step_begin();
-  extern __shared__ __align__(16) int32_t s_off[];  // [planes * kSub + 1], or the dense step's columns
+  extern __shared__ int32_t s_off[];  // [planes * kSub + 1]
   const int R = d.n_bins, planes = d.bin_hi - d.bin_lo + 1;
   const ScatterScratch ws0 = scatter_scratch(d, 0);
   __shared__ int32_t s_spk;
@@ -1078,8 +1079,8 @@ __global__ void __launch_bounds__(kEngThreads, MS <= 4 ? 4 : 3) k_eng_scatter_fl
     int q = si.q_t - d.bin_lo;
     if (q < 0) q += R + 1;
     long long ev = 0, ed = 0;
-    __syncthreads();  // the offsets have been read: their memory takes the columns
-    scatter_dense<MS>(d, scatter_scratch(d, q), reinterpret_cast<float(*)[32][32]>(s_off), ev, ed);
+    __shared__ float s_acc[kEngThreads / 32][32][32];  // (beside the offsets: overlaid on them, 1.4 % slower at 20 bins)
+    scatter_dense<MS>(d, scatter_scratch(d, q), s_acc, ev, ed);
     if (d.stats) block_stats(d, k, ev, ed);
     return;
   }
@@ -2012,14 +2013,15 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int planes = d.bin_hi - d.bin_lo + 1;
     const int ms = mask_stride(d.batch);
+    // Shared memory of a block: the offsets of all planes (33 KB at 128 bins) beside the
+    // 33 KB of a dense step's columns; from 60 planes on more than a kernel has without
+    // an attribute, from 92 on three blocks fit an SM instead of four.
+    const size_t ssmem = sizeof(int32_t) * size_t(planes * kSub + 1);
+    const size_t sblock = ssmem + kScatterStatic + 1024;  // (1 KB of every block is the system's)
     // one wave of resident blocks, fewer when the step cannot list that many rows
     const int64_t rows_per_block = d.scatter_lanes == 1 ? 64 : d.scatter_lanes == 8 ? kEngThreads / 8 : kEngThreads / 32;
-    const int64_t wave = int64_t(sms) * (ms <= 4 ? 4 : 3);
+    const int64_t wave = int64_t(sms) * std::min<int64_t>(ms <= 4 ? 4 : 3, int64_t(228 * 1024 / sblock));
     const unsigned sgrid = unsigned(std::max<int64_t>(1, std::min(wave, ceil_div(n * planes, rows_per_block))));
-    // the offsets of all planes, or the columns of a dense step, which has one plane:
-    // at most 33 KB (128 bins), within the 48 KB that need no attribute
-    const size_t ssmem = std::max(sizeof(int32_t) * size_t(planes * kSub + 1),
-                                  d.dense_rows > 0 ? sizeof(float) * (kEngThreads / 32) * 32 * 32 : size_t(0));
     // every divisor a power of two or a verified reciprocal: no IEEE division compiled in
     const bool fast = fast_divisors(d, KIND);
     auto neuron = fast ? (S == 1 ? k_eng_neuron<KIND, HARD, USE_REF, 1, true>
@@ -2050,14 +2052,18 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
                                                                                              : k_eng_scatter_rows<8>;
     const int64_t columns = d.dense_rows > 0 ? int64_t(kRowWarps) * 32 * 32 : 0;
     const size_t rsmem = sizeof(float) * size_t(kRowList + std::max(n, columns));
+    // dynamic shared memory beyond what a kernel has without asking: its range's most, once
+    auto allow = [&](const void* kern, size_t most) {
+      if (launch_setup_known(kern, dev, most, 1)) return int(BT_OK);
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)) != cudaSuccess)
+        return bt_set_error(BT_ERR_CUDA, "shared memory request of %zu bytes refused", most);
+      launch_setup_add(kern, dev, most, 1);
+      return int(BT_OK);
+    };
     if (parts) {
-      const void* kern = reinterpret_cast<const void*>(rows);
-      const size_t most = sizeof(float) * size_t(kRowList + kRowMaxN);
-      if (!launch_setup_known(kern, dev, most, 1)) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)) != cudaSuccess)
-          return bt_set_error(BT_ERR_CUDA, "shared memory request of %zu bytes refused", most);
-        launch_setup_add(kern, dev, most, 1);
-      }
+      if (int st = allow(reinterpret_cast<const void*>(rows), sizeof(float) * size_t(kRowList + kRowMaxN))) return st;
+    } else if (ssmem + kScatterStatic > 48 * 1024) {
+      if (int st = allow(reinterpret_cast<const void*>(scatter), sizeof(int32_t) * size_t(BT_MAX_BINS * kSub + 1))) return st;
     }
     for (int64_t k = 0; k < d.n_steps; ++k) {
       const StepIdx si = step_idx(d.t0 + k, d.n_bins, d.hist_len);
