@@ -12,8 +12,8 @@
 namespace bt {
 
 // spmm.cu: out [batch][n_rows] from gT [n_cols][pitch], as a step kernel
-int rows_product(int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* ptr, const uint32_t* col, const float* wts,
-                 const float* gT, float* out, cudaStream_t s);
+int rows_product(bool first, int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* ptr, const uint32_t* col,
+                 const float* wts, const float* gT, float* out, cudaStream_t s);
 
 struct BpttStep {
   const float *x, *psc, *v, *ref, *gk, *z;        // drive and state before the step, its spikes
@@ -211,7 +211,7 @@ extern "C" int bt_bptt_backward(const bt_bptt_desc* d, void* stream) {
   k_bptt_begin<<<grid, 256, 0, s>>>(B, pitch, n, d->cur_psc, row(d->g_psc, T - 1), d->G_psc + (T - 1) * per, d->gT);
   BT_CHECK_LAUNCH("k_bptt_begin");
   for (int64_t t = T - 1; t >= 0; --t) {
-    if (int st = rows_product(B, pitch, n, d->csr_ptr, d->csr_dst, d->csr_w, d->gT, d->gz, s)) return st;
+    if (int st = rows_product(false, B, pitch, n, d->csr_ptr, d->csr_dst, d->csr_w, d->gT, d->gz, s)) return st;
     BpttStep a;
     a.x = d->x + t * per;
     a.psc = d->psc + t * per;
@@ -230,7 +230,7 @@ extern "C" int bt_bptt_backward(const bt_bptt_desc* d, void* stream) {
     a.g_I = d->G_I + t * per;
     a.next_psc = t > 0 ? d->G_psc + (t - 1) * per : d->cur_psc;
     a.next_T = t > 0 ? d->gT : nullptr;
-    if (launch_step(kern, grid, 256, 0, s, nd, d->psc_coef, d->psc_tau, B, pitch, n, int(d->detach_reset), a) != cudaSuccess)
+    if (launch_step(false, kern, grid, 256, 0, s, nd, d->psc_coef, d->psc_tau, B, pitch, n, int(d->detach_reset), a) != cudaSuccess)
       break;
   }
   BT_CHECK_LAUNCH("k_bptt_step");

@@ -185,13 +185,23 @@ inline void launch_setup_add(const void* kern, int dev, size_t smem, int blocks)
 // it), so its launch latency and the set-up of its blocks overlap the other's
 // tail; step_begin then waits for that grid to complete and its writes to be
 // visible before any global access.
+// A block may thus be resident while the launch before its own, and even the
+// one before that, still writes.  So:
+//  - the first launch of a chain is an ordinary one (first): all that was
+//    written before the chain is complete when any of its blocks starts, and
+//    may be read through the read-only path and ahead of the wait;
+//  - what a launch of the chain writes (state, spike sets and lists, transposed
+//    operands, packed weights) is read by the later ones through plain pointers:
+//    no __restrict__, __ldg, __ldcg or ld.global.nc, whose loads need data that
+//    does not change while the kernel is resident and are not ordered after
+//    the wait.
 __device__ __forceinline__ void step_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <typename... P, typename... A>
-cudaError_t launch_step(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+cudaError_t launch_step(bool first, void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(unsigned(threads));
@@ -201,7 +211,7 @@ cudaError_t launch_step(void (*kern)(P...), dim3 grid, int threads, size_t smem,
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = first ? 0 : 1;
   return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 

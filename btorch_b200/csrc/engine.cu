@@ -273,12 +273,12 @@ __global__ void __launch_bounds__(kEngThreads) k_eng_neuron(bt_engine_desc d, in
   const bool valid = i < n;
   const int nb = B - b0 < S ? B - b0 : S;  // samples of this block (uniform)
   const int off0 = b0 * n + (valid ? i : 0);
-  float* __restrict__ ring_p = d.ring + off0;  // acc: W z of the previous step
-  float* __restrict__ psc_p = d.psc + off0;
-  float* __restrict__ v_p = d.v + off0;
-  float* __restrict__ ref_p = USE_REF ? d.refractory + off0 : nullptr;
-  float* __restrict__ gk_p = KIND == BT_NEURON_ALIF ? d.g_k + off0 : nullptr;
-  const float* __restrict__ x_p = d.x ? d.x + int64_t(k) * B * n + off0 : nullptr;
+  float* ring_p = d.ring + off0;  // acc: W z of the previous step
+  float* psc_p = d.psc + off0;
+  float* v_p = d.v + off0;
+  float* ref_p = USE_REF ? d.refractory + off0 : nullptr;
+  float* gk_p = KIND == BT_NEURON_ALIF ? d.g_k + off0 : nullptr;
+  const float* x_p = d.x ? d.x + int64_t(k) * B * n + off0 : nullptr;
   const uint64_t pol_stream = l2_evict_first(), pol_keep = l2_evict_last();
   // Every load before the first store: a load behind a store through a
   // pointer that may alias it waits for the store.  A sample past its length
@@ -628,8 +628,8 @@ __global__ void __launch_bounds__(kEngThreads) k_eng_neuron_rec(bt_engine_desc d
   const bool st_traces = d.v_trace || d.psc_trace || d.ref_trace || d.gk_trace;
   if (i < n && (k <= len || st_traces)) {  // else: past its length, nothing to read or write
     const int64_t idx = b * n + i, c0 = b * nc + i * C;
-    float* __restrict__ ring = d.ring + c0;
-    float* __restrict__ psc = d.psc + c0;
+    float* ring = d.ring + c0;
+    float* psc = d.psc + c0;
     // loads
     float pend[M], stv[M], pc[M], pt[M];
     if constexpr (CT == 4) {
@@ -1227,9 +1227,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_eng_scatter_rows(bt_engine_d
   const int w0 = tid * per < words ? tid * per : words, w1 = w0 + per < words ? w0 + per : words;
   int h = si.h_t - bin;
   if (h < 0) h += d.hist_len;
-  const uint32_t* bits = d.hist + (int64_t(h) * B + b) * words;
+  const uint32_t* bits = d.hist + (int64_t(h) * B + b) * words;  // (this step's words: plain loads)
   int cnt = 0;
-  for (int w = w0; w < w1; ++w) cnt += __popc(__ldcg(bits + w));
+  for (int w = w0; w < w1; ++w) cnt += __popc(bits[w]);
   for (int i = tid; i < n; i += kRowThreads) acc[i] = 0.0f;
   int incl = cnt;
 #pragma unroll
@@ -1251,7 +1251,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_eng_scatter_rows(bt_engine_d
     const int rows = own1 - base < kRowList ? own1 - base : kRowList;
     int at = first - base;
     for (int w = w0; w < w1; ++w) {
-      uint32_t m = __ldcg(bits + w);
+      uint32_t m = bits[w];
       while (m) {
         const int l = __ffs(m) - 1;
         m &= m - 1;
@@ -2068,12 +2068,12 @@ int run_typed(const bt_engine_desc& d, const float* z_given, cudaStream_t s) {
     for (int64_t k = 0; k < d.n_steps; ++k) {
       const StepIdx si = step_idx(d.t0 + k, d.n_bins, d.hist_len);
       // nothing runs on after a refused launch: the state would move on without its input
-      cudaError_t e = C > 1 ? launch_step(rec, rgrid, kEngThreads, 0, s, d, k, si)
-                      : vec ? launch_step(nvec, vgrid, kVecThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given)
-                            : launch_step(neuron, grid, kEngThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
+      cudaError_t e = C > 1 ? launch_step(k == 0, rec, rgrid, kEngThreads, 0, s, d, k, si)
+                      : vec ? launch_step(k == 0, nvec, vgrid, kVecThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given)
+                            : launch_step(k == 0, neuron, grid, kEngThreads, 0, s, d, int(k), si, scatter_scratch(d, si.q_t), z_given);
       if (e == cudaSuccess)
-        e = parts ? launch_step(rows, dim3(unsigned(d.batch * parts)), kRowThreads, rsmem, s, d, si, parts)
-                  : launch_step(scatter, dim3(sgrid), kEngThreads, ssmem, s, d, k, si);
+        e = parts ? launch_step(false, rows, dim3(unsigned(d.batch * parts)), kRowThreads, rsmem, s, d, si, parts)
+                  : launch_step(false, scatter, dim3(sgrid), kEngThreads, ssmem, s, d, k, si);
       if (e != cudaSuccess) break;
     }
     BT_CHECK_LAUNCH("k_eng_neuron/k_eng_scatter");

@@ -36,17 +36,17 @@ struct FVec {
   float v[V];
 };
 
+// Plain loads: the transposed operand is written by the launches before, which
+// may still run when this one's blocks start (launch_step).
 template <int V>
 __device__ __forceinline__ FVec<V> ld_vec(const float* p) {
   FVec<V> r;
   if constexpr (V == 4) {
-    const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 q = *reinterpret_cast<const float4*>(p);
     r.v[0] = q.x, r.v[1] = q.y, r.v[2] = q.z, r.v[3] = q.w;
-  } else if constexpr (V == 2) {
-    const float2 q = __ldg(reinterpret_cast<const float2*>(p));
-    r.v[0] = q.x, r.v[1] = q.y;
   } else {
-    r.v[0] = __ldg(p);
+    static_assert(V == 1, "runs of 4 samples or single ones");
+    r.v[0] = *p;
   }
   return r;
 }
@@ -73,7 +73,7 @@ constexpr int kGatherUnroll = 8;
 template <int V, int G, int P, bool SKIP0>
 __device__ __forceinline__ void rows_gather(int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* __restrict__ ptr,
                                             const uint32_t* __restrict__ col, const float* __restrict__ wts,
-                                            const float* __restrict__ gT, float* __restrict__ out) {
+                                            const float* gT, float* out) {
   constexpr int S = 32 / G, R = kGatherWarps / P;  // lane groups of a warp, rows of a CTA
   __shared__ float s_out[kGatherWarps][G * V + 1];
   const int warp = int(threadIdx.x >> 5), lane = int(lane_id());
@@ -140,8 +140,8 @@ template <int V, int G, int P>
 __global__ void __launch_bounds__(kGatherWarps * 32, 4) k_rows_gather(int64_t batch, int64_t pitch, int64_t n_rows,
                                                                   const int32_t* __restrict__ ptr,
                                                                   const uint32_t* __restrict__ col,
-                                                                  const float* __restrict__ wts,
-                                                                  const float* __restrict__ gT, float* __restrict__ out) {
+                                                                  const float* __restrict__ wts, const float* gT,
+                                                                  float* out) {
   step_begin();
   rows_gather<V, G, P, false>(batch, pitch, n_rows, ptr, col, wts, gT, out);
 }
@@ -175,11 +175,12 @@ static void pick_lanes(int64_t pitch, int64_t n_rows, F&& go) {
 }
 
 // out [batch][n_rows] from gT [n_cols][pitch] (pitch >= batch, zeros past it).
-int rows_product(int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* ptr, const uint32_t* col,
+// first: no launch of the caller's goes before it (launch_step).
+int rows_product(bool first, int64_t batch, int64_t pitch, int64_t n_rows, const int32_t* ptr, const uint32_t* col,
                  const float* wts, const float* gT, float* out, cudaStream_t s) {
   auto go = [&](auto v, auto g, auto p, int64_t ny) {
     constexpr int V = decltype(v)::value, G = decltype(g)::value, P = decltype(p)::value;
-    launch_step(k_rows_gather<V, G, P>, dim3(unsigned(ceil_div(n_rows, kGatherWarps / P)), unsigned(ny)),
+    launch_step(first, k_rows_gather<V, G, P>, dim3(unsigned(ceil_div(n_rows, kGatherWarps / P)), unsigned(ny)),
                 kGatherWarps * 32, 0, s, batch, pitch, n_rows, ptr, col, wts, gT, out);
   };
   // scratch that is not padded to a multiple of 4, or not aligned, is read in words
@@ -244,8 +245,7 @@ __global__ void __launch_bounds__(256) k_compact(int64_t total, const float* __r
 __global__ void __launch_bounds__(256) k_push_prepare(int64_t batch, int64_t n_in, int64_t n_out, int64_t pitch,
                                                       int64_t nnz, const float* __restrict__ x,
                                                       const int32_t* __restrict__ perm, const float* __restrict__ w,
-                                                      const int32_t* __restrict__ ctl, float* __restrict__ scratch,
-                                                      float* __restrict__ out) {
+                                                      const int32_t* ctl, float* scratch, float* out) {
   step_begin();
   __shared__ float tile[32][33];
   if (push_dense(ctl, n_in, pitch)) {
@@ -287,10 +287,9 @@ __global__ void __launch_bounds__(256) k_push_prepare(int64_t batch, int64_t n_i
 template <int V, int G, int P>
 __global__ void __launch_bounds__(kGatherWarps * 32, 3) k_push_product(
     int64_t batch, int64_t n_in, int64_t n_out, int64_t pitch, const int32_t* __restrict__ csr_ptr,
-    const uint32_t* __restrict__ csr_dst, const float* __restrict__ csr_w, const int32_t* __restrict__ csc_ptr,
-    const uint32_t* __restrict__ csc_src, const float* __restrict__ w, const float* __restrict__ x,
-    const int32_t* __restrict__ ctl, const int32_t* __restrict__ list, const float* __restrict__ xT,
-    float* __restrict__ out) {
+    const uint32_t* __restrict__ csr_dst, const float* csr_w, const int32_t* __restrict__ csc_ptr,
+    const uint32_t* __restrict__ csc_src, const float* __restrict__ w, const float* __restrict__ x, const int32_t* ctl,
+    const int32_t* list, const float* xT, float* out) {
   step_begin();
   if (push_dense(ctl, n_in, pitch)) {
     rows_gather<V, G, P, true>(batch, pitch, n_out, csc_ptr, csc_src, w, xT, out);
@@ -337,7 +336,7 @@ int grad_input_t(int64_t batch, int64_t pitch, int64_t n_in, int64_t n_out, cons
     k_transpose<<<tgrid, dim3(32, 8), 0, s>>>(batch, n_out, pitch, grad_out, work);
     BT_CHECK_LAUNCH("k_transpose");
   }
-  return rows_product(batch, pitch, n_in, csr_ptr, csr_dst, csr_w, work, grad_x, s);
+  return rows_product(n_out == 0, batch, pitch, n_in, csr_ptr, csr_dst, csr_w, work, grad_x, s);
 }
 }  // namespace
 
@@ -397,13 +396,13 @@ extern "C" int bt_spmv_push(int64_t batch, int64_t n_in, int64_t n_out, int64_t 
   BT_CHECK_LAUNCH("k_compact");
   const int64_t most = std::max(std::max(ceil_div(batch * n_out, 1024), ceil_div(nnz, 1024)),
                                 ceil_div(n_in, 32) * ceil_div(pitch, 32));
-  launch_step(k_push_prepare, dim3(unsigned(std::min<int64_t>(148 * 8, most))), 256, 0, s, batch, n_in, n_out, pitch, nnz,
+  launch_step(false, k_push_prepare, dim3(unsigned(std::min<int64_t>(148 * 8, most))), 256, 0, s, batch, n_in, n_out, pitch, nnz,
               x, csr_w ? nullptr : csr_perm, w, work, scratch, out);
   BT_CHECK_LAUNCH("k_push_prepare");
   const float* packed = csr_w ? csr_w : scratch;
   pick_lanes<4>(pitch, n_out, [&](auto v, auto g, auto p, int64_t ny) {
     constexpr int V = decltype(v)::value, G = decltype(g)::value, P = decltype(p)::value;
-    launch_step(k_push_product<V, G, P>, dim3(unsigned(ceil_div(n_out, kGatherWarps / P)), unsigned(ny)),
+    launch_step(false, k_push_product<V, G, P>, dim3(unsigned(ceil_div(n_out, kGatherWarps / P)), unsigned(ny)),
                 kGatherWarps * 32, 0, s, batch, n_in, n_out, pitch, csr_ptr, csr_dst, packed, csc_ptr, csc_src, w, x, work,
                 list, scratch, out);
   });
