@@ -262,12 +262,13 @@ __global__ void k_transpose_dense(int64_t rows, int64_t cols, int64_t pitch, con
 
 using namespace bt;
 
-// work: 8 control words, the lists, then (dense_rows) the transposed input
+// work: 8 control words, the lists of one pass, then the transposed input of a
+// batch that fits one pass (longer ones never take the dense path)
 extern "C" int64_t bt_grad_weight_work_words(int64_t rows, int64_t n_in, int32_t with_dense) {
   if (rows < 0 || n_in < 0) return 0;
   const int64_t seg = rows < kGwSegment ? rows : kGwSegment;
   int64_t words = 8 + n_in * gw_stride(seg) / 2;
-  if (with_dense) words += n_in * (ceil_div(rows, 4) * 4);
+  if (with_dense && rows <= kGwSegment) words += n_in * (ceil_div(rows, 4) * 4);
   return words;
 }
 
