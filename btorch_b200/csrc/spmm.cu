@@ -353,40 +353,31 @@ extern "C" int bt_spmv_grad_input_pad(int64_t batch, int64_t n_in, int64_t n_out
                       stream);
 }
 
+// Samples of one pass of bt_spmv_push, whose scratch holds two arrays of x's size (the
+// list of its nonzeros, and x transposed where the gather runs): all of them while
+// an array stays within 256 MB; beyond that as many as keep it there, or half of
+// them up to 512, whose two arrays take no more than one of the whole batch.  (A pass
+// that pushes packs the weights again, 12 bytes an edge: below 512 samples that
+// starts to show.)  Sample blocks are the grid's y: below 2^22 samples.
+static int64_t push_samples(int64_t batch, int64_t n_in) {
+  constexpr int64_t kWords = int64_t(1) << 26, kSlab = int64_t(1) << 22;
+  const int64_t half = std::min<int64_t>(ceil_div(batch, 2), 512);
+  const int64_t most = std::min(kSlab, std::max(kWords / std::max<int64_t>(n_in, 1), half));
+  return std::min(batch, std::max<int64_t>(4, most & ~int64_t(3)));
+}
+
 // work: 8 control words, the list of nonzeros, then x transposed or the packed weights
 extern "C" int64_t bt_spmv_push_work_words(int64_t batch, int64_t n_in, int64_t padded) {
   if (batch < 0 || n_in < 0 || padded < 0) return 0;
-  const int64_t pitch = ceil_div(batch, 4) * 4;
-  return 8 + ceil_div(batch * n_in, 4) * 4 + std::max(pitch * n_in, ceil_div(padded, 4) * 4);
+  const int64_t samples = push_samples(batch, n_in), pitch = ceil_div(samples, 4) * 4;
+  return 8 + ceil_div(samples * n_in, 4) * 4 + std::max(pitch * n_in, ceil_div(padded, 4) * 4);
 }
 
-extern "C" int bt_spmv_push(int64_t batch, int64_t n_in, int64_t n_out, int64_t nnz, const int32_t* csr_ptr,
-                            const uint32_t* csr_dst, const int32_t* csr_perm, const float* csr_w, const int32_t* csc_ptr,
-                            const uint32_t* csc_src, const float* w, const float* x, float* out, int32_t* work,
-                            void* stream) {
-  BT_CHECK_ARG(batch >= 0 && n_in >= 0 && n_out >= 0 && nnz >= 0, "negative size");
-  BT_CHECK_ARG(batch * n_in < (int64_t(1) << 31), "batch * n_in must be below 2^31");
-  if (batch == 0 || n_out == 0) return BT_OK;
-  // sample blocks are the grid's y (below 65536): larger batches go in slabs, one
-  // after the other through the same scratch
-  constexpr int64_t kSlab = int64_t(1) << 22;
-  if (batch > kSlab) {
-    for (int64_t b0 = 0; b0 < batch; b0 += kSlab)
-      if (int st = bt_spmv_push(std::min(kSlab, batch - b0), n_in, n_out, nnz, csr_ptr, csr_dst, csr_perm, csr_w, csc_ptr,
-                                csc_src, w, x ? x + b0 * n_in : nullptr, out ? out + b0 * n_out : nullptr, work, stream))
-        return st;
-    return BT_OK;
-  }
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  BT_CHECK_ARG(out, "null pointer");
-  if (n_in == 0 || nnz == 0) {
-    if (cudaMemsetAsync(out, 0, sizeof(float) * size_t(batch * n_out), s) != cudaSuccess)
-      return bt_set_error(BT_ERR_CUDA, "memset failed");
-    return BT_OK;
-  }
-  BT_CHECK_ARG(csr_ptr && csr_dst && (csr_perm || csr_w) && csc_ptr && csc_src && w && x && work, "null pointer");
-  BT_CHECK_ARG(((reinterpret_cast<uintptr_t>(csr_dst) | reinterpret_cast<uintptr_t>(csr_w) |
-                 reinterpret_cast<uintptr_t>(work)) & 15) == 0, "edge arrays and work must be 16-byte aligned");
+namespace {
+// One pass, of push_samples samples at most.
+int push_pass(int64_t batch, int64_t n_in, int64_t n_out, int64_t nnz, const int32_t* csr_ptr, const uint32_t* csr_dst,
+              const int32_t* csr_perm, const float* csr_w, const int32_t* csc_ptr, const uint32_t* csc_src, const float* w,
+              const float* x, float* out, int32_t* work, cudaStream_t s) {
   const int64_t pitch = ceil_div(batch, 4) * 4, total = batch * n_in;
   int32_t* list = work + 8;
   float* scratch = reinterpret_cast<float*>(work + 8 + ceil_div(total, 4) * 4);
@@ -407,5 +398,31 @@ extern "C" int bt_spmv_push(int64_t batch, int64_t n_in, int64_t n_out, int64_t 
                 list, scratch, out);
   });
   BT_CHECK_LAUNCH("k_push_product");
+  return BT_OK;
+}
+}  // namespace
+
+extern "C" int bt_spmv_push(int64_t batch, int64_t n_in, int64_t n_out, int64_t nnz, const int32_t* csr_ptr,
+                            const uint32_t* csr_dst, const int32_t* csr_perm, const float* csr_w, const int32_t* csc_ptr,
+                            const uint32_t* csc_src, const float* w, const float* x, float* out, int32_t* work,
+                            void* stream) {
+  BT_CHECK_ARG(batch >= 0 && n_in >= 0 && n_out >= 0 && nnz >= 0, "negative size");
+  BT_CHECK_ARG(batch * n_in < (int64_t(1) << 31), "batch * n_in must be below 2^31");
+  if (batch == 0 || n_out == 0) return BT_OK;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  BT_CHECK_ARG(out, "null pointer");
+  if (n_in == 0 || nnz == 0) {
+    if (cudaMemsetAsync(out, 0, sizeof(float) * size_t(batch * n_out), s) != cudaSuccess)
+      return bt_set_error(BT_ERR_CUDA, "memset failed");
+    return BT_OK;
+  }
+  BT_CHECK_ARG(csr_ptr && csr_dst && (csr_perm || csr_w) && csc_ptr && csc_src && w && x && work, "null pointer");
+  BT_CHECK_ARG(((reinterpret_cast<uintptr_t>(csr_dst) | reinterpret_cast<uintptr_t>(csr_w) |
+                 reinterpret_cast<uintptr_t>(work)) & 15) == 0, "edge arrays and work must be 16-byte aligned");
+  const int64_t samples = push_samples(batch, n_in);
+  for (int64_t b0 = 0; b0 < batch; b0 += samples)  // one after the other through the same scratch
+    if (int st = push_pass(std::min(samples, batch - b0), n_in, n_out, nnz, csr_ptr, csr_dst, csr_perm, csr_w, csc_ptr,
+                           csc_src, w, x + b0 * n_in, out + b0 * n_out, work, s))
+      return st;
   return BT_OK;
 }

@@ -130,7 +130,8 @@ BT_API int bt_spmv_scatter(int64_t batch, int64_t n_in, int64_t n_out,
  * from x transposed (a fixed tree of fmaf chains per output, zero inputs
  * skipped).  w: weights in canonical order; csr_w: the same in CSR order
  * (padded like csr_dst), or NULL with csr_perm, which packs them when the push
- * runs.  csr_dst padded to a multiple of 4.  `work`:
+ * runs.  csr_dst padded to a multiple of 4.  Long batches go in passes through
+ * the same scratch.  `work`:
  * bt_spmv_push_work_words(batch, n_in, length of csr_dst) int32 words, 16-byte
  * aligned. */
 BT_API int64_t bt_spmv_push_work_words(int64_t batch, int64_t n_in, int64_t padded);
