@@ -42,6 +42,7 @@ order (tests compare both with the reference's autograd within 1e-4).
 from __future__ import annotations
 
 import ctypes as CT
+import time
 
 import torch
 import torch.nn as nn
@@ -56,6 +57,21 @@ from .neurons.lif import LIF
 from .synapse import ExponentialPSC
 
 MEMORY_FRACTION = 0.25  # largest share of free device memory the step buffers may take
+FREE_AGE = 0.5  # seconds for which a figure of the free memory serves calls far below it
+_FREE: dict = {}  # device -> (when, free bytes) as last asked for
+
+
+def fits(device, need: int) -> bool:
+    """`need` bytes are at most MEMORY_FRACTION of the free device memory.
+    Asking the driver takes up to milliseconds, as long as a small call: one
+    that needs less than a sixteenth of what is allowed goes by a figure up to
+    FREE_AGE seconds old."""
+    when, free = _FREE.get(device, (float("-inf"), 0))
+    now = time.monotonic()
+    if now - when > FREE_AGE or 16 * need > MEMORY_FRACTION * free:
+        free = torch.cuda.mem_get_info(device)[0]
+        _FREE[device] = (now, free)
+    return need <= MEMORY_FRACTION * free
 
 
 def match(rnn) -> tuple[dict | None, str]:
@@ -491,9 +507,10 @@ class _FusedBPTT(torch.autograd.Function):
         return g_x, g_w, g_b, g_mag, cur_v, g_psc, cur_gk, None, None, None, None
 
 
-def _bytes_needed(T, B, n, C, kinds, has_gk, has_ref, proj, c_in, native):
+def _bytes_needed(T, B, n, C, kinds, has_gk, has_ref, proj, c_in, native, nnz=0):
     """Device bytes of the call's buffers (spikes, stacks, step buffers,
-    chunk-start states, gradients of one chunk)."""
+    chunk-start states, gradients of one chunk, the weight gradient's row
+    lists, the edges packed for the forward and the backward)."""
     n_ch = -(-T // C)
     ckpt = n_ch > 1
     Cb = C if ckpt else T
@@ -503,7 +520,8 @@ def _bytes_needed(T, B, n, C, kinds, has_gk, has_ref, proj, c_in, native):
     per += 0 if native else 4 * Cb  # I, u, mask, v_charged
     per += states * (n_ch if ckpt else 0)  # chunk-start states
     per += Cb if native and ckpt and proj else 2 * Cb  # gradients of a chunk (dI over its drive)
-    return 4 * B * n * per + (4 * Cb * B * (2 * c_in + 1) if proj else 0)
+    lists = L.lib().bt_grad_weight_work_words(Cb * B, n, 0)
+    return 4 * (B * n * per + (Cb * B * (2 * c_in + 1) if proj else 0) + lists + 3 * nnz)
 
 
 def run(rnn, x: torch.Tensor, paths: dict):
@@ -528,11 +546,8 @@ def run(rnn, x: torch.Tensor, paths: dict):
     C = checkpoint_chunk(rnn, T)
     kinds = frozenset(paths.values())
     need = _bytes_needed(T, B, n, C, kinds, isinstance(neuron, ALIF), neuron._use_refractory, inp is not None, c_in,
-                         native_steps(rnn, B, n, syn.linear.direction(B)))
-    # (asking the driver for the free memory costs up to milliseconds: only for
-    # calls of a size that matters)
-    total = torch.cuda.get_device_properties(x.device).total_memory
-    if need > total // 64 and need > MEMORY_FRACTION * torch.cuda.mem_get_info(x.device)[0]:
+                         native_steps(rnn, B, n, syn.linear.direction(B)), int(syn.linear.indices.shape[1]))
+    if not fits(x.device, need):
         return None
     shape = v.shape
     v0 = v.reshape(B, n)
@@ -540,7 +555,11 @@ def run(rnn, x: torch.Tensor, paths: dict):
     gk0 = neuron.g_k.reshape(B, n) if isinstance(neuron, ALIF) else None
     ref0 = neuron.refractory.reshape(B, n).detach() if neuron._use_refractory else None
     syn.linear._edge_weight()  # one weight per stored nonzero, or an error before any launch
-    outs = _FusedBPTT.apply(xin, w_in, b_in, syn.linear.magnitude, v0, psc0, gk0, ref0, rnn, kinds, C)
+    try:
+        outs = _FusedBPTT.apply(xin, w_in, b_in, syn.linear.magnitude, v0, psc0, gk0, ref0, rnn, kinds, C)
+    except torch.OutOfMemoryError:  # (the free memory was less than the figure; no state has changed)
+        _FREE.pop(x.device, None)
+        return None
     Z, Vst, Pst, GKst, REFst, vT, pT, gT, rT = outs
     neuron.v = vT.reshape(shape)
     syn.psc = pT.reshape(syn.psc.shape)
