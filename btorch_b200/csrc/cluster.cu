@@ -32,6 +32,9 @@
 // read of the copy (its step k - 1 reads steps k - 2 .. k - 1 - R).  With
 // delay bins the copies of the call's first steps' history come from the
 // history ring (d.hist) at the start.
+// A wait that runs into its limit sets a flag in every CTA: nothing waits, is
+// published or arrives from then on, the CTAs meet behind the loop, account for
+// the words sent and wait for the last of them to land before any CTA exits.
 // After the last step the launch applies the synapse update of that step
 // (the gather engine's final launch) and writes the state back: one launch
 // per call, nothing per step in global memory but the input read and the
@@ -117,6 +120,18 @@ __device__ __forceinline__ void mbar_arm(uint64_t* bar, uint32_t bytes) {
                : "memory");
   (void)state;
 }
+// counts `bytes` as arrived that no copy or store will bring
+__device__ __forceinline__ void mbar_complete(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t count) {
+  uint64_t state;
+  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 %0, [%1], %2;"
+               : "=l"(state)
+               : "r"(smem_addr(bar)), "r"(count)
+               : "memory");
+  (void)state;
+}
 // phase with this parity complete? (acquire at cluster scope: the remote
 // stores it counted are visible)
 __device__ __forceinline__ bool mbar_done(uint64_t* bar, uint32_t parity) {
@@ -198,6 +213,12 @@ struct ClusterTile {
   unsigned spin;
 };
 
+// What a lane and a CTA did before a wait gave up, for the drain behind the loop.
+struct ClusterDone {
+  unsigned sent[2] = {0u, 0u};  // words this lane sent to CTA `lane`, by step parity (lane = rank: arrivals)
+  int armed;                    // thread 0: the barriers are armed for the steps below this one
+};
+
 // The time loop when every (word, sample) item of a tile has a warp of its own
 // and every divisor is fast.  The item's state stays in registers, its
 // addresses advance by additions, and the warps wait for a step's words each by
@@ -208,7 +229,8 @@ struct ClusterTile {
 // instructions per warp and step outside the in-edge walk (16 rows: 2.26 us a
 // step, 96 rows 3.1), which is what this one shortens.
 template <int KIND, bool HARD, bool USE_REF, int IDS>
-__device__ __forceinline__ void cluster_one(const bt_engine_desc& d, const ClusterTile& t, cg::cluster_group& cluster) {
+__device__ __forceinline__ void cluster_one(const bt_engine_desc& d, const ClusterTile& t, cg::cluster_group& cluster,
+                                            ClusterDone& done) {
   constexpr bool SRC16 = IDS == 0, DELAY = IDS == 2, ALIF = KIND == BT_NEURON_ALIF;
   using G4 = typename SrcGroup<SRC16>::T;
   constexpr int NG = kClRows / 4;
@@ -238,6 +260,7 @@ __device__ __forceinline__ void cluster_one(const bt_engine_desc& d, const Clust
   int h_t = int(d.t0 % t.H);
   const int deg = t.s_deg[l];
   float x_ahead = (xp && valid && 0 < len) ? __ldcs(xp) : 0.0f;
+  int stop = 0;               // steps this lane published
   int kc = 0, kp = t.Hc - 1;  // the copies of steps k and k - 1
   for (int k = 0; k <= steps; ++k) {
     G4 sn[NG];
@@ -267,7 +290,10 @@ __device__ __forceinline__ void cluster_one(const bt_engine_desc& d, const Clust
       __syncwarp();
       // armed for step k + 1 before this warp publishes step k, which every sender
       // of step k + 1 has to have received
-      if (threadIdx.x == 0 && !*t.dead && k + 1 < steps) mbar_arm(bar, t.expect);
+      if (threadIdx.x == 0 && !*t.dead && k + 1 < steps) {
+        mbar_arm(bar, t.expect);
+        done.armed = k + 2;
+      }
       if (k - 1 < len) {
         const char* base = reinterpret_cast<const char*>(t.s_bits) + uint32_t(b * t.Wd) * 4u;
         const char* bits = base + uint32_t(kp) * cstride;
@@ -330,14 +356,16 @@ __device__ __forceinline__ void cluster_one(const bt_engine_desc& d, const Clust
     }
     const uint32_t word = __ballot_sync(0xffffffffu, valid && s != 0.0f);
     const uint32_t off = uint32_t(kc) * cstride;
+    // nothing is sent or arrives once a wait gave up: the phase may never complete then
+    // (no arming arrival, no bytes), and an arrival beyond its count is a fault
+    const bool gone = *t.dead != 0;
     if (lane == t.rank) {
       *reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(t.s_bits) + off0 + off) = word;
-      // not once a wait gave up: the phase may never complete then (no arming
-      // arrival, no bytes), and an arrival beyond its count is a fault
-      if (!*t.dead) mbar_arrive(t.s_mbar + (k & 1));
-    } else if (remote && !*t.dead) {
+      if (!gone) mbar_arrive(t.s_mbar + (k & 1));
+    } else if (remote && !gone) {
       st_async_word(rbits + off, word, rbar + uint32_t(k & 1) * 8u);
     }
+    if (!gone) stop = k + 1;
     if (traces && valid) {
       if (d.v_trace) d.v_trace[tix] = v;
       if (USE_REF && d.ref_trace) d.ref_trace[tix] = ref;
@@ -367,6 +395,7 @@ __device__ __forceinline__ void cluster_one(const bt_engine_desc& d, const Clust
   t.s_v[q] = v;
   t.s_ref[q] = ref;
   t.s_gk[q] = gk;
+  if (lane < t.CL) done.sent[0] = unsigned(stop + 1) >> 1, done.sent[1] = unsigned(stop) >> 1;
 }
 
 // ONE: cluster_one's time loop (every item has a warp, fast divisors).
@@ -460,7 +489,10 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
   // a wait gave up somewhere in the cluster: every CTA stops waiting and
   // publishing, runs out its loop and meets the others at the final barrier
   __shared__ int s_dead;
+  __shared__ unsigned s_sent[2], s_arrived[2];  // drain: words sent to this CTA, its own warps' arrivals, by step parity
   volatile int* dead = &s_dead;
+  ClusterDone done;
+  done.armed = int(d.n_steps < 2 ? d.n_steps : 2);
   const uint32_t expect = uint32_t(4 * B * (words - NWv));
   if (threadIdx.x == 0) {
     // ONE: own warps' arrivals beside the arming one
@@ -468,6 +500,7 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
     mbar_init(&s_mbar[1], ONE ? 1u + unsigned(NWv * B) : 1u);
     mbar_init_fence();
     s_dead = 0;
+    s_sent[0] = s_sent[1] = s_arrived[0] = s_arrived[1] = 0u;
     mbar_arm(&s_mbar[0], expect);
     if (d.n_steps > 1) mbar_arm(&s_mbar[1], expect);
   }
@@ -493,7 +526,7 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
     const ClusterTile t{B,    Tp,  Wd,    words, w0,    tile_n, NWv,    R,     Hc,    H,     rank,   CL,    n,
                         p0,   s_v, s_psc, s_ref, s_gk,  s_w,    s_src,  s_bits, s_gptr, s_len, s_deg,  s_mbar, dead,
                         &s_dead, expect, spin};
-    if (warp < NWv * B) cluster_one<KIND, HARD, USE_REF, IDS>(d, t, cluster);
+    if (warp < NWv * B) cluster_one<KIND, HARD, USE_REF, IDS>(d, t, cluster, done);
   } else {
   const int items = NWv * B;  // (word, sample) pairs of this tile; item it = (b, w) = divmod(it, NWv)
   int h_t = int(d.t0 % H);
@@ -520,7 +553,10 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
             break;
           }
         }
-        if (!*dead && k + 1 < d.n_steps) mbar_arm(&s_mbar[prv], expect);  // for step k + 1
+        if (!*dead && k + 1 < d.n_steps) {
+          mbar_arm(&s_mbar[prv], expect);  // for step k + 1
+          done.armed = int(k + 2);
+        }
       }
       __syncthreads();  // also orders this CTA's own words (plain stores) before they are read
     }
@@ -610,7 +646,11 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
       // publish: lane c stores the word into CTA c's copy (c = rank: its own)
       const int off = (kc * B + b) * Wd + w0 + w;
       if (lane == rank) s_bits[off] = word;
-      else if (lane < CL && !*dead) st_async_word(cluster_addr(s_bits + off, lane), word, cluster_addr(&s_mbar[cur], lane));
+      else if (lane < CL && !*dead) {
+        st_async_word(cluster_addr(s_bits + off, lane), word, cluster_addr(&s_mbar[cur], lane));
+        if (cur) ++done.sent[1];
+        else ++done.sent[0];
+      }
       if (s != 0.0f) {
         st_ev += s_deg[l];
         st_un += 1;
@@ -666,8 +706,32 @@ __global__ void __launch_bounds__(kClThreadsMax, 1) k_cluster_engine(bt_engine_d
   // wait covers the last step); the barrier keeps every CTA resident until
   // all have left the loop, also when a wait gave up
   cluster.sync();
-  // words still under way when the others stopped waiting land before any CTA exits
-  if (*dead) __nanosleep(20000u);
+  if (*dead) {
+    // A wait gave up (the same answer in every CTA: the flag's stores precede the
+    // setter's arrival).  Words may still be under way to a CTA, which must not exit
+    // before they land, and the barrier does not order st.async.  Every sender tells
+    // how many words it sent; the receiver completes its phases by what was armed but
+    // never sent, so that they end when the last word has landed, and waits for that
+    // (within a limit, as for its own bulk copies).
+    if (lane < CL) {
+      unsigned* to = lane != rank ? cluster.map_shared_rank(&s_sent[0], lane) : &s_arrived[0];
+      if (done.sent[0]) atomicAdd(to + 0, done.sent[0]);
+      if (done.sent[1]) atomicAdd(to + 1, done.sent[1]);
+    }
+    cluster.sync();
+    if (threadIdx.x == 0) {
+      for (int p = 0; p < 2; ++p) {
+        const unsigned phases = unsigned(done.armed + 1 - p) >> 1;  // armed steps of this parity
+        if (!phases) continue;
+        const uint32_t never = phases * expect - 4u * s_sent[p];
+        if (never) mbar_complete(&s_mbar[p], never);
+        const uint32_t late = ONE ? phases * uint32_t(NWv * B) - s_arrived[p] : 0u;
+        if (late) mbar_arrive_n(&s_mbar[p], late);
+        for (unsigned polls = 0; !mbar_done(&s_mbar[p], (phases - 1u) & 1u) && polls < kClDefaultSpinLimit;) ++polls;
+      }
+      for (unsigned polls = 0; !mbar_done(&s_mbar[2], 0) && polls < kClDefaultSpinLimit;) ++polls;
+    }
+  }
   for (int q = threadIdx.x; q < B * Tp; q += T) {
     const int b = q / Tp, l = q - b * Tp;
     if (l >= tile_n) continue;
