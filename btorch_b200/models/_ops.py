@@ -242,7 +242,7 @@ def sparse_mm(x2d, w_canon, layout, direction, w_csr=None):
     L.require_cuda(x2d, w_canon, what="SparseConn")
     if x2d.dtype != torch.float32 or w_canon.dtype != torch.float32:
         raise TypeError("SparseConn supports float32 only.")
-    x2d = x2d.contiguous()
+    x2d, w_canon = x2d.contiguous(), w_canon.contiguous()  # (the kernels index both as one run)
     if torch.is_grad_enabled() and (x2d.requires_grad or w_canon.requires_grad):
         return SparseMM.apply(x2d, w_canon, layout, direction, w_csr)
     return _spmv(direction, layout, x2d, w_canon.detach(), w_csr)
