@@ -225,9 +225,10 @@ def _memory_var(rv: ResetValue, batch_size, **fmt) -> torch.Tensor:
         device = fmt.get("device")
         if device is not None and torch.device(device).type != "cpu" and np.ndim(rv.value) == 0 \
                 and not (torch.is_tensor(rv.value) and rv.value.is_cuda):
-            # a scalar is filled in on the device (a copy from the host would wait for the stream)
-            t = torch.as_tensor(rv.value)
-            return torch.full(sizes, t.item(), dtype=fmt.get("dtype") or t.dtype, device=device)
+            # a scalar, converted on the host, is filled in on the device (a copy from the host
+            # would wait for the stream)
+            t = torch.as_tensor(rv.value, dtype=fmt.get("dtype"))
+            return torch.full(sizes, t.detach().item(), dtype=t.dtype, device=device)
         v = torch.as_tensor(rv.value, **fmt).detach().clone()
     if tuple(v.shape) != sizes:
         v = torch.broadcast_to(v, sizes).clone()
