@@ -143,6 +143,10 @@ class SpikeHistory(MemoryModule):
                 cursor, self.history = None, torch.empty_like(self.history)
             L.check(L.lib().bt_history_store(batch, self.max_delay, self.size, ring.data_ptr(), t_end, H, cursor,
                                              advance, self.history.data_ptr(), s), "bt_history_store")
+            if self.use_circular_buffer:  # written in place: as the tensor moves below, a new version
+                written = [t for t in (self.history, self._cursor) if not t.is_inference()]
+                if written:
+                    torch.autograd.graph.increment_version(written)
             return
         block = torch.empty((self.max_delay, batch, self.size), device=ring.device, dtype=torch.float32)
         sel = torch.stack([ring[(t_end - 1 - d) % H] for d in range(self.max_delay)]).contiguous()
