@@ -93,7 +93,21 @@ def heuristic(conn, batch: int, receptors: int = 1) -> EngineChoice:
     return EngineChoice(mode)
 
 
-def candidates(conn, batch: int, receptors: int = 1, n_bins: int = 1, n: int = 0, dev=None) -> list[EngineChoice]:
+def aligned(plan, rnn, x) -> bool:
+    """The arrays of a neuron step start on 16 bytes: always those of a
+    captured graph, which are its own, and those the engine allocates."""
+    if rnn.cudagraph:
+        return True
+    node = plan.neuron
+    own = [node.v, plan.psc_mod.psc, getattr(node, "refractory", None), getattr(node, "g_k", None)]
+    if plan.inp is None and x.is_cuda and x.is_contiguous():
+        own.append(x)
+    return all(t.data_ptr() % 16 == 0 for t in own if torch.is_tensor(t))
+
+
+def candidates(conn, batch: int, receptors: int = 1, n_bins: int = 1, n: int = 0, dev=None,
+               vectors: bool = True) -> list[EngineChoice]:
+    """vectors: the state's arrays admit 16-byte accesses (aligned)."""
     out = []
     mw = L.lib().bt_mask_stride(batch)
     modes = allowed_modes(conn, batch, receptors, n_bins)
@@ -119,9 +133,9 @@ def candidates(conn, batch: int, receptors: int = 1, n_bins: int = 1, n: int = 0
                     out.append(EngineChoice(mode, tile_posts=0 if mult == 1 else tp))
             continue
         if mode == L.BT_MODE_SCATTER:
-            # (n a multiple of 4 without receptor channels: the vectorised neuron
-            # step, whatever spt)
-            for spt in (1, 2, 4) if n % 4 or receptors > 1 or n == 0 else (1,):
+            # (n a multiple of 4 without receptor channels, aligned state: the
+            # vectorised neuron step, whatever spt)
+            for spt in (1, 2, 4) if n % 4 or receptors > 1 or n == 0 or not vectors else (1,):
                 if spt > 1 and spt > batch:
                     continue
                 for lanes in (1, 8, 32):
@@ -157,7 +171,8 @@ def choose(plan, rnn, x: torch.Tensor, sample_len, run) -> EngineChoice:
         return cache[key][0]
     if not plan.conn.sparse_config.autotune or T < TUNE_MIN_STEPS:
         return heuristic(plan.conn, B, plan.n_rec)
-    cands = candidates(plan.conn, B, plan.n_rec, plan.n_bins, plan.neuron.size, plan.neuron.v.device)
+    cands = candidates(plan.conn, B, plan.n_rec, plan.n_bins, plan.neuron.size, plan.neuron.v.device,
+                       aligned(plan, rnn, x))
     if plan.uniform_delay:  # a DelayedPSC delay: the tile mode has none
         cands = [c for c in cands if c.mode != L.BT_MODE_TILE]
     if len(cands) == 1:
