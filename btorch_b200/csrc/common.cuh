@@ -142,6 +142,17 @@ __device__ __forceinline__ void red_add_f32(float* ptr, float v, uint64_t pol) {
   asm volatile("red.global.add.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(ptr), "f"(v), "l"(pol));
 }
 
+// SMs of the current device.
+inline int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    (void)cudaGetLastError();
+    return 148;
+  }
+  return sms;
+}
+
 // Launch set-ups already checked (kernel, device, dynamic shared memory,
 // blocks): the attribute calls and occupancy queries of a persistent launch
 // run once per set-up, not on every call -- they cost the host far more

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 4) k_rows_gather(int64_t ba
 template <int V, int G, typename F>
 static void pick_parts(int64_t pitch, int64_t n_rows, F&& go) {
   const int64_t ny = ceil_div(pitch, G * V);
-  const int64_t warps = n_rows * ny, want = 148 * 40;
+  const int64_t warps = n_rows * ny, want = int64_t(device_sms()) * 40;
   using std::integral_constant;
   const integral_constant<int, V> v;
   const integral_constant<int, G> g;
@@ -387,7 +387,7 @@ int push_pass(int64_t batch, int64_t n_in, int64_t n_out, int64_t nnz, const int
   BT_CHECK_LAUNCH("k_compact");
   const int64_t most = std::max(std::max(ceil_div(batch * n_out, 1024), ceil_div(nnz, 1024)),
                                 ceil_div(n_in, 32) * ceil_div(pitch, 32));
-  launch_step(false, k_push_prepare, dim3(unsigned(std::min<int64_t>(148 * 8, most))), 256, 0, s, batch, n_in, n_out, pitch, nnz,
+  launch_step(false, k_push_prepare, dim3(unsigned(std::min<int64_t>(device_sms() * 8, most))), 256, 0, s, batch, n_in, n_out, pitch, nnz,
               x, csr_w ? nullptr : csr_perm, w, work, scratch, out);
   BT_CHECK_LAUNCH("k_push_prepare");
   const float* packed = csr_w ? csr_w : scratch;

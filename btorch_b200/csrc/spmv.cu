@@ -187,7 +187,7 @@ static inline int grid_for_warps(int64_t warps, int threads = 256) {
 // Ordered gather: warps per output until about 64 per SM are in flight (one
 // warp walking 16 samples of 2000 outputs in turn leaves the chip idle).
 static inline dim3 gather_grid(int64_t n_out, int64_t batch) {
-  int64_t y = ceil_div(148 * 64, n_out);
+  int64_t y = ceil_div(int64_t(device_sms()) * 64, n_out);
   if (y > batch) y = batch;
   return dim3(unsigned(grid_for_warps(n_out)), unsigned(y < 1 ? 1 : y));
 }
@@ -228,10 +228,7 @@ extern "C" int bt_spmv_scatter(int64_t batch, int64_t n_in, int64_t n_out, const
   if (total == 0) return BT_OK;
   k_compact_nonzero<<<int(ceil_div(total, 256)), 256, 0, s>>>(total, x, work);
   BT_CHECK_LAUNCH("k_compact_nonzero");
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  k_spmv_scatter<<<sms * 8, 256, 0, s>>>(n_in, n_out, csr_ptr, csr_dst, csr_w, x, work, out);
+  k_spmv_scatter<<<device_sms() * 8, 256, 0, s>>>(n_in, n_out, csr_ptr, csr_dst, csr_w, x, work, out);
   BT_CHECK_LAUNCH("k_spmv_scatter");
   return BT_OK;
 }
