@@ -37,6 +37,13 @@ class Kept:
                 t.record_stream(cur)  # (the keeper may let go of it while this stream still reads)
         return self.arrays
 
+    def __reduce__(self):  # a copy of the keeper starts without (copy.deepcopy, pickle)
+        return _nothing, ()
+
+
+def _nothing():
+    return None
+
 
 def keepable() -> bool:
     return not torch.cuda.is_current_stream_capturing()

@@ -117,3 +117,22 @@ def test_runs_on_two_streams(mode):
                 got.append(rnn(x, engine_choice=choice)[0])
         torch.cuda.synchronize()
     assert torch.equal(got[0], want) and torch.equal(got[1], want)
+
+
+def test_a_copied_connection_starts_without_kept_arrays():
+    import copy
+
+    m, dense = conn(5, grad=True)
+    x = (torch.rand((16, 700), device=DEV) < 0.1).float().requires_grad_(True)
+    g = torch.ones((16, 700), device=DEV)
+    torch.autograd.grad(m(x), x, g)  # keeps the packed weights
+    twin = copy.deepcopy(m)
+    with torch.no_grad():
+        twin.magnitude.mul_(2.0)
+    assert torch.equal(torch.autograd.grad(twin(x), x, g)[0], 2.0 * (g @ dense.T))
+    assert torch.equal(torch.autograd.grad(m(x), x, g)[0], g @ dense.T)
+    rnn = net(640, 1, direction="auto")
+    z = torch.ones((3, 1, 640), device=DEV) * 3.0
+    with torch.no_grad(), environ.context(dt=1.0):
+        rnn(z, engine_choice=EngineChoice(L.BT_MODE_CLUSTER))
+    assert copy.deepcopy(rnn.synapse.linear)._cluster_packed is None
