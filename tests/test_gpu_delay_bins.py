@@ -76,3 +76,24 @@ def test_one_plane_with_and_without_dense_steps(lanes, dense, delay, n, batch):
     x[1::7] = 16.0  # steps in which most neurons fire in every sample
     compare(make, x, batch, lambda rnn: (rnn.synapse.psc_module if delay else rnn.synapse).psc, scatter_lanes=lanes,
             dense_rows=dense)
+
+
+@pytest.mark.parametrize("batch,every", [(1, 1), (1, 3), (33, 1)])
+def test_more_rows_than_one_pass_takes(batch, every):
+    """Bursts that list more rows than the grid's warps take at once (32 each): several passes, equal shares."""
+    n, bins, T = 16384, 20, 26
+    rng = np.random.default_rng(7)
+    pre, post, delay = (rng.integers(0, k, 40 * n) for k in (n, n, bins))
+    key = np.unique((pre * bins + delay) * n + post)
+    w = (rng.integers(1, 5, key.size) * 2.0**-8).astype(np.float32)
+    m = sp.coo_array((w, (key // n, key % n)), shape=(n * bins, n))
+    rti = pd.DataFrame({"receptor_type": ["syn"], "receptor_index": [0]})
+
+    def make():
+        conn = SparseConn(m, enforce_dale=False, sparse_config={"direction": "scatter"})
+        syn = HeterSynapsePSC(n, 1, rti, conn, max_delay_steps=bins, use_circular_buffer=True, tau_syn=5.0)
+        return RecurrentNN(LIF(n, hard_reset=True), syn, update_state_names=("neuron.v",)).cuda()
+
+    x = torch.zeros((T, batch, n), device="cuda")
+    x[:, :, ::every] = 32.0  # they fire in every step
+    compare(make, x, batch, lambda rnn: rnn.synapse.base_psc.psc, scatter_lanes=1)
