@@ -435,13 +435,21 @@ __device__ __forceinline__ void neuron_update4(const NeuronParams& pr, const flo
 // otherwise every lane appends its own.  Called by every lane of the warp.
 __device__ __forceinline__ void publish_nibble(const ScatterScratch& ws, int i0, int b, uint32_t nib) {
   const unsigned lane = lane_id();
-  uint32_t first = 0;
+  // The four neurons' mask bits are all issued before the first result is looked at.
+  // The first spike in a word of the mask asks the flag whether it is the neuron's
+  // first; a mask of one word needs none.
+  uint32_t was[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q)
-    if (nib & (1u << q)) {
-      atomicOr(ws.mask + int64_t(i0 + q) * ws.ms + (b >> 5), 1u << (b & 31));
-      if (atomicOr(ws.flag + i0 + q, 1) == 0) first |= 1u << q;
-    }
+    was[q] = nib & (1u << q) ? atomicOr(ws.mask + int64_t(i0 + q) * ws.ms + (b >> 5), 1u << (b & 31)) : 1u;
+  if (ws.ms > 1) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (was[q] == 0u) was[q] = uint32_t(atomicOr(ws.flag + i0 + q, 1));
+  }
+  uint32_t first = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) first |= (was[q] == 0u ? 1u : 0u) << q;
   const int cnt = __popc(first), nspk = __popc(nib);
   int64_t at;
   if (ws.cap_shift >= 7) {
