@@ -264,7 +264,7 @@ __device__ __forceinline__ void publish_spikes(const bt_engine_desc& d, const St
 template <int KIND, bool HARD, bool USE_REF, int S, bool FAST>
 __global__ void __launch_bounds__(kEngThreads) k_eng_neuron(bt_engine_desc d, int k, StepIdx si, ScatterScratch ws,
                                                           const float* __restrict__ z_given) {
-  step_begin();
+  step_wait();
   const int n = int(d.n), B = int(d.batch);
   const int words = (n + 31) >> 5;
   const int i = int(blockIdx.x) * kEngThreads + int(threadIdx.x);
@@ -493,7 +493,7 @@ constexpr int kVecThreads = 128;
 template <int KIND, bool HARD, bool USE_REF, bool FAST>
 __global__ void __launch_bounds__(kVecThreads) k_eng_neuron_vec(bt_engine_desc d, int k, StepIdx si, ScatterScratch ws,
                                                                 const float* __restrict__ z_given) {
-  step_begin();
+  step_wait();
   const int n = int(d.n), B = int(d.batch);
   const int words = (n + 31) >> 5;
   const int i0 = (int(blockIdx.x) * kVecThreads + int(threadIdx.x)) * 4;

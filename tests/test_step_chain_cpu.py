@@ -16,14 +16,14 @@ def chain_kernels():
     out = []
     for path in sorted(CSRC.glob("*.cu")):
         for m in KERNEL.finditer(path.read_text()):
-            if "step_begin();" in m.group(3):
+            if re.search(r"step_(begin|wait)\(\);", m.group(3)):
                 out.append(pytest.param(m.group(2), m.group(3), id=m.group(1)))
     return out
 
 
 def test_every_chain_kernel_is_seen():
     text = "".join(p.read_text() for p in CSRC.glob("*.cu"))
-    assert len(chain_kernels()) == text.count("step_begin();") >= 9
+    assert len(chain_kernels()) == len(re.findall(r"step_(?:begin|wait)\(\);", text)) >= 9
 
 
 @pytest.mark.parametrize("params,body", chain_kernels())
