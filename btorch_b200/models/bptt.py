@@ -180,9 +180,9 @@ def native_steps(rnn, B: int, n: int, direction: str) -> bool:
 
 
 class _Run:
-    """The engine as the forward of a BPTT call: scatter or ordered gather, one
-    delay bin, state in this object's own [B][n] buffers, successive `steps`
-    calls continuing one run."""
+    """The engine as the forward of a BPTT call: scatter or ordered (a warp per
+    neuron, "gather", or a lane, "pull"), one delay bin, state in this object's
+    own [B][n] buffers, successive `steps` calls continuing one run."""
 
     def __init__(self, neuron, d, psc_mod, coef, tau, lay, direction, w, B, n, v, psc, gk, ref):
         dev = w.device
@@ -205,8 +205,19 @@ class _Run:
         hist = torch.zeros((3, B, (n + 31) // 32), device=dev, dtype=torch.int32)
         e.hist = hist.data_ptr()
         self.keep.append(hist)
-        self.gather = direction == "gather"
-        if self.gather:
+        self.ordered = direction in ("gather", "pull")
+        if direction == "pull":
+            e.mode = L.BT_MODE_PULL
+            sl = getattr(lay, "slices", None)
+            if sl is None:
+                sl = lay.slices = _ops.build_slices(lay, dev)
+            sl_w = _ops.pack_slice_weights(sl, w)
+            masks = torch.zeros((3, n + 1, L.lib().bt_mask_stride(B)), device=dev, dtype=torch.int32)
+            self.keep += [sl, sl_w, masks]
+            e.sl_ptr, e.sl_src, e.sl_w = sl.sl_ptr.data_ptr(), sl.sl_src.data_ptr(), sl_w.data_ptr()
+            e.masks = masks.data_ptr()
+            return
+        if direction == "gather":
             e.mode = L.BT_MODE_GATHER
             e.csc_ptr, e.csc_src, e.csc_w = lay.csc_ptr.data_ptr(), lay.csc_src.data_ptr(), w.data_ptr()
             return
@@ -237,7 +248,7 @@ class _Run:
         e = self.desc
         e.x, e.n_steps, e.spikes = x.data_ptr(), kc, L.ptr(spikes)
         e.v_trace, e.psc_trace, e.gk_trace, e.ref_trace = L.ptr(v), L.ptr(psc), L.ptr(gk), L.ptr(ref)
-        if given is not None and not self.gather:
+        if given is not None and not self.ordered:
             L.check(L.lib().bt_engine_run_given(CT.byref(e), given.data_ptr(), s), "bt_engine_run_given")
         else:
             L.check(L.lib().bt_engine_run(CT.byref(e), s), "bt_engine_run")
@@ -316,7 +327,11 @@ class _FusedBPTT(torch.autograd.Function):
                       "gk": new(n_ch, B, n) if gk0 is not None else None,
                       "ref": new(n_ch, B, n) if ref0 is not None else None}
         if native:
-            run = _Run(neuron, d, psc_mod, coef, tau, lay, direction, w, B, n, v0, psc0, gk0, ref0)
+            # (the engine's own choice for the ordered modes: a warp per neuron walks the
+            # samples one after the other)
+            engine = "pull" if direction == "gather" and B >= conn.sparse_config.pull_min_batch else direction
+            run = _Run(neuron, d, psc_mod, coef, tau, lay, engine, w, B, n, v0, psc0, gk0, ref0)
+            ctx.engine = engine
             st = None if ckpt else _Traces(B, n, T, gk0 is not None, ref0 is not None, proj, c_in, dev)
             out = new(Cb, B, n) if proj and ckpt else None
             pw = _projection_scratch(Cb, B, c_in, dev) if out is not None else None
@@ -435,7 +450,7 @@ class _FusedBPTT(torch.autograd.Function):
                 if ckpt:
                     start = [t[ci] if t is not None else None for t in map(ctx.bounds.get, ("v", "psc", "gk", "ref"))]
                     if run is None:
-                        run = _Run(None, d, ctx, ctx.coef, ctx.tau, lay, ctx.direction, w, B, n, *start)
+                        run = _Run(None, d, ctx, ctx.coef, ctx.tau, lay, ctx.engine, w, B, n, *start)
                     else:
                         run.load(*start)
                     st.start(run)
