@@ -98,11 +98,11 @@ __global__ void __launch_bounds__(512) k_active_rows(int64_t r0, int64_t seg, in
 // (row-minor, post stride = 4 mod 32 words: the 32-byte row segments are
 // stored without conflicts).  A list's first 16 bytes carry its count and 7
 // rows, so a source that is mostly silent costs one sector; byte offsets and
-// the padding keep an entry at four instructions (201 us with a test and an
-// index computation per entry, 125 without, at 3.3M edges, 2560 rows, 1.2 %
-// spikes; 1210 us when every edge walked the samples' mask words and read the
-// gradient from global memory).  Bound by L1 (91 %): the random shared-memory
-// reads, 2.7 wavefronts each, and the lists' scattered vectors.
+// the padding keep an entry at four instructions (3.3M edges, 2560 rows, 1 %
+// spikes: 149 us; a test and an index computation per entry took 1.6 times as
+// long, and 1210 us when every edge walked the samples' mask words and read the
+// gradient from global memory).  Bound by L1 (84 % of peak): the random
+// shared-memory reads (18M wavefronts) and the lists' scattered vectors.
 // carry: continue the chain from grad_w (a later row segment); add: add the
 // chain's total to grad_w (a later chunk).
 __global__ void __launch_bounds__(kGwThreads) k_grad_weight_lists(int64_t r0, int64_t seg, int64_t rows, int64_t n_in,

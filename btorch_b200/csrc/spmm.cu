@@ -53,7 +53,8 @@ __device__ __forceinline__ FVec<V> ld_vec(const float* p) {
 
 constexpr int kGatherWarps = 8;
 // Runs of gT in flight per lane (8: 4200 rows of 410 edges at batch 128 68 us, 88
-// with the 4 the compiler kept in flight; 64 registers, no spills).
+// with the 4 the compiler kept in flight; at the 64 registers of four blocks the
+// widest instances spill 4 to 24 bytes).
 constexpr int kGatherUnroll = 8;
 
 // G lanes (a power of two) cover a block of G V samples at V samples each; the
